@@ -151,18 +151,23 @@ __device__ __forceinline__ void rain_cell(const Phys& P, int cid, float dt, cons
 struct DSum {
     float S1, S2, T;
 };
-__device__ __forceinline__ void dsum_add(DSum& s, float r2, float rho_j, const FF& rr) {
+__device__ __forceinline__ void dsum_add_if(DSum& s, float r2, float rho_j, const FF& rr, bool near) {
     // accepted pairs only (r2 < 4): the spline of w3 in Horner form with FMAs,
     // scaled by 4 / SIGMA_W (4 - 6 q^2 + 3 q^3 inside, (2 - q)^3 outside): the
     // epilogue uses the sums only as the ratios S1 / S2 and T / S2
     const float q = r2 * rsqrt_normal(fmaxf(r2, 1e-30f));   // 0 at r2 = 0
     const float t = 2.0f - q;
-    const float W = q < 1.0f ? __fmaf_rn(q * q, __fmaf_rn(3.0f, q, -6.0f), 4.0f) : t * t * t;
-    const float rj = fmaxf(rho_j, 1e-3f);
+    const float Wq = q < 1.0f ? __fmaf_rn(q * q, __fmaf_rn(3.0f, q, -6.0f), 4.0f) : t * t * t;
+    // what is not near adds exact zeros, whatever its fields hold
+    const float W = near ? Wq : 0.f;
+    const float rj = near ? fmaxf(rho_j, 1e-3f) : 1.0f;
     const float iw = W * rcp_normal(rj);
     s.S1 += W;
     s.S2 += iw;
     s.T = fmaf(iw, rj - rr.hi, s.T);   // rho_ref's low part enters once, in the epilogue
+}
+__device__ __forceinline__ void dsum_add(DSum& s, float r2, float rho_j, const FF& rr) {
+    dsum_add_if(s, r2, rho_j, rr, true);
 }
 
 // Density result + EOS + saturation adjustment + autoconversion (+ Kessler

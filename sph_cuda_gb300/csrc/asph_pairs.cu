@@ -13,15 +13,20 @@
 // excluded) in a slot-major list; M walks that list.
 //
 // D, brick path.  One CTA per Morton-aligned brick of BX x BY x BZ cells;
-// the brick's targets are one contiguous span of the sorted order and the
-// block has about as many threads as a brick has targets.  The CTA copies
-// the particles of every table cell within H cells of the brick into shared
-// memory, bucketed row-major by region cell, so that each row of a target's
-// 5 x 5 x 5 window is one contiguous span of shared memory; each thread
-// walks its target's row spans in one flattened loop, queues accepted
-// candidates in a small per-thread list in shared memory, and drains the
-// list (density sums + neighbour-list writes) in uniform loops.  H = 2 (the
-// stencil) covers every target still in a cell of its brick; H = 3 also
+// the brick's targets are one contiguous span of the sorted order, a thread
+// each.  The CTA copies the particles of every table cell within H cells of the
+// brick into shared memory, bucketed row-major by region cell, so that each
+// row of a target's 5 x 5 x 5 window is one contiguous span of slots.  A
+// warp walks its targets' rows together, two candidates a step in fp16, queues
+// what that test passes in a small per-thread list in shared memory, and
+// drains the lists (float test, density sums, neighbour-list writes) together.
+// What bounds the pass is instruction issue: about 75 candidates and 20
+// neighbours per target at 0.6 particles per cell against 48 bytes.  Density per
+// step at 2M, walk in float with a row advance in every step against this one:
+// 0.6 per cell 511 -> 470 us, the same clustered 1018 -> 830 us, 8:1 cells
+// 516 -> 448 us, one per cell 620 -> 438 us (there with the smaller brick and
+// halo too); 475k 152 -> 135 us, 262k at one per cell 206 -> 147 us.
+// H = 2 (the stencil) covers every target still in a cell of its brick; H = 3 also
 // covers one cell of drift since the sort.  A region that overflows the
 // staging capacity is split into its two Morton-aligned halves (each a
 // contiguous sub-span of the targets with a smaller region), and a half
@@ -38,6 +43,7 @@
 // memory, the reference's loop structure; used for grids narrower than the
 // staged region, and by M for a target whose list overflowed or was not
 // produced on the current positions.
+#include <cuda_fp16.h>
 #include "asph_device.cuh"
 #include "../../include/asph.h"
 
@@ -46,6 +52,14 @@ namespace asph {
 constexpr int MAX_HALO = 3;      // widest staged halo (cells around a brick)
 constexpr int DENSITY_REGS = 48; // register cap of the brick kernel (its launch plan counts on it)
 constexpr int DLIST = 30;        // most queued accepted candidates per thread (D); a launch may use fewer
+// The walk's fp16 test of a candidate.  Coordinates are within FCLAMP < 8
+// cells of the region's centre, so their fp16 rounding is at most 2^-9 each
+// (plus 1e-4 from forming them in float), a pair's distance is off by less than
+// 2 sqrt(3) (2^-9 + 1e-4) = 0.0072, a pair with r < 2 has a rounded r^2 below
+// 4.029, and the five fp16 roundings of forming it (2^-11 relative each) leave
+// it below 4.0389.  The threshold is the next fp16 number above.
+constexpr float FCLAMP = 7.9f;
+constexpr float FTHR = 4.0390625f;
 // Momentum blocks of 128 threads: a block ends with its slowest warp, and
 // smaller blocks waste less of an SM on warps that wait for it (measured at
 // 2M from init: 0.298 / 0.260 / 0.257 / 0.271 ms at 32 / 64 / 128 / 256).
@@ -89,7 +103,8 @@ struct BrickHalves {
 struct PairCfg {
     int nbx, nby, nbz, nbricks;
     int cap;            // staged particles that fit in shared memory
-    int dlist;          // drain-queue depth of this launch (<= DLIST; queues drain above dlist - 4)
+    int dlist;          // drain-queue depth of this launch (16 to DLIST)
+    uint32_t qinv;      // 2^32 / bytes of a queue row, rounded up
 };
 
 namespace {
@@ -157,15 +172,6 @@ __device__ __forceinline__ void for_window_global(const Phys& P, const int2* __r
         }
 }
 
-// Span of one window row (cells ix-2 .. ix+2) inside the staged region.
-// (Culling the span geometrically with a drift bound was measured slower at
-// 0.6 particles per cell: the per-row arithmetic costs more than the candidates it
-// removes.)
-__device__ __forceinline__ void row_span(const int* s_off, int la_m2, int& k, int& kend) {
-    k = s_off[la_m2];
-    kend = s_off[la_m2 + 2 * STENCIL + 1];
-}
-
 // Region-local window of a target: returns false if it leaves the region.
 template <int BX, int BY, int BZ, int H>
 __device__ __forceinline__ bool local_window(const Phys& P, int ox, int oy, int oz, float x, float y, float z,
@@ -185,63 +191,60 @@ __device__ __forceinline__ bool local_window(const Phys& P, int ox, int oy, int 
 
 // Offsets of the staged region of a brick: s_off[l] = first slot of region
 // cell l (row-major, H cells around the brick, x/y wrapped), s_off[R] =
-// the total, s_start[l] = the cell's first global index, and (when it fits,
-// total <= cap) s_gidx[k] = the global index of slot k.  A cell's particles
-// take consecutive slots in index order.  The cell-table loads are strided
-// over the block with four in flight per thread; the scan runs in shared
-// memory.
+// the total, and s_gidx[k] = the global index of every slot that fits.  A
+// cell's particles take consecutive slots in index order.  Two threads take a row of cells, half of it each, all their table
+// loads in flight: the threads' order is the slots' order, so one block scan
+// of the threads' counts gives the offsets.
 template <int BX, int BY, int BZ, int H>
 __device__ int region_offsets(const Phys& P, const int2* __restrict__ range, int ox, int oy, int oz, int* s_off,
-                              int* s_start, int* s_gidx, int cap, int* s_warp) {
+                              int* s_gidx, int cap, int* s_warp) {
     using G = BrickGeom<BX, BY, BZ, H>;
+    constexpr int HX = G::RX / 2, HALVES = 2 * G::RY * G::RZ;
     const int T = blockDim.x;
-    const int rx0 = ox - H, ry0 = oy - H, rz0 = oz - H;
-    for (int lb = threadIdx.x; lb < G::R; lb += 4 * T) {
-        int2 rg[4];
+    int carry = 0;
+    for (int q0 = 0; q0 < HALVES; q0 += T) {
+        const int q = q0 + threadIdx.x, row = q >> 1, x0 = (q & 1) * HX;
+        int start[HX], cnt[HX];
+        const int lz = row / G::RY, ly = row - lz * G::RY, gz = oz - H + lz;
+        int gy = oy - H + ly;
+        gy += gy < 0 ? P.ny : 0; gy -= gy >= P.ny ? P.ny : 0;
+        const bool in = q < HALVES && gz >= 0 && gz < P.nz;
+        const int2* const tab = range + (size_t)(gz * P.ny + gy) * P.nx;
+        int run = 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int l = lb + u * T;
-            rg[u] = make_int2(0, 0);
-            if (l < G::R) {
-                const int lx = l % G::RX, ly = (l / G::RX) % G::RY, lz = l / (G::RX * G::RY);
-                const int gz = rz0 + lz;
-                if (gz >= 0 && gz < P.nz) {
-                    int gx = rx0 + lx, gy = ry0 + ly;
-                    gx += gx < 0 ? P.nx : 0; gx -= gx >= P.nx ? P.nx : 0;
-                    gy += gy < 0 ? P.ny : 0; gy -= gy >= P.ny ? P.ny : 0;
-                    rg[u] = range[(size_t)(gz * P.ny + gy) * P.nx + gx];
-                }
-            }
+        for (int c = 0; c < HX; ++c) {
+            int gx = ox - H + x0 + c;
+            gx += gx < 0 ? P.nx : 0; gx -= gx >= P.nx ? P.nx : 0;
+            const int2 rg = in ? tab[gx] : make_int2(0, 0);
+            start[c] = rg.x;
+            cnt[c] = rg.y - rg.x;
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int l = lb + u * T;
-            if (l < G::R) {
-                s_start[l] = rg[u].x;
-                s_off[l] = rg[u].y - rg[u].x;
+        for (int c = 0; c < HX; ++c) run += cnt[c];
+        int total;
+        int k = carry + block_excl_scan_int(run, s_warp, &total);
+        carry += total;
+        if (q < HALVES) {
+            int* const o = s_off + row * G::RX + x0;
+#pragma unroll
+            for (int c = 0; c < HX; ++c) {
+                o[c] = k;
+                const int e = min(cnt[c], cap - k);   // slots beyond the capacity: the region is split
+                for (int j = 0; j < e; ++j) s_gidx[k + j] = start[c] + j;
+                k += cnt[c];
             }
         }
     }
+    if (threadIdx.x == 0) s_off[G::R] = carry;
     __syncthreads();
-    const int chunk = (G::R + T - 1) / T;
-    const int l0 = threadIdx.x * chunk, l1 = min(l0 + chunk, G::R);
-    int run = 0;
-    for (int l = l0; l < l1; ++l) run += s_off[l];
-    int total;
-    int excl = block_excl_scan_int(run, s_warp, &total);
-    const bool map = total <= cap;
-    for (int l = l0; l < l1; ++l) {
-        const int c = s_off[l];
-        s_off[l] = excl;
-        if (map) {
-            const int g = s_start[l];
-            for (int k = 0; k < c; ++k) s_gidx[excl + k] = g + k;
-        }
-        excl += c;
-    }
-    if (threadIdx.x == 0) s_off[G::R] = total;
-    __syncthreads();
-    return total;
+    return carry;
+}
+
+__device__ __forceinline__ uint32_t h2_bits(__half2 h) { return *reinterpret_cast<uint32_t*>(&h); }
+__device__ __forceinline__ __half2 h2_of(uint32_t b) { return *reinterpret_cast<__half2*>(&b); }
+// fp16 cell coordinate from the region's centre.  Clamping brings points together, never apart.
+__device__ __forceinline__ __half feat_coord(float x, float c, float inv) {
+    return __float2half_rn(fminf(fmaxf((x - c) * inv, -FCLAMP), FCLAMP));
 }
 
 // Neighbour-list writer of one target (slot-major, coalesced over targets).
@@ -256,6 +259,19 @@ struct NbrOut {
             p += N;
         }
         ++n;
+    }
+    __device__ __forceinline__ void push_if(bool take, int j) {   // predicated, no branch
+        asm volatile("{\n"
+                     "  .reg .pred p, q;\n"
+                     "  setp.ne.s32 p, %2, 0;\n"
+                     "  setp.lt.and.s32 q, %1, %4, p;\n"
+                     "  @q st.global.u32 [%0], %3;\n"
+                     "  @q add.u64 %0, %0, %5;\n"
+                     "  @p add.s32 %1, %1, 1;\n"
+                     "}\n"
+                     : "+l"(p), "+r"(n)
+                     : "r"((int)take), "r"(j), "n"(NBR_CAP), "l"(N * 4)
+                     : "memory");
     }
 };
 
@@ -319,13 +335,15 @@ __global__ __launch_bounds__(256) void k_density_global(const __grid_constant__ 
     density_eos_epilogue(P, A.out, i, pi, s, rr, dt);
 }
 
-// Pointers into the density pass's dynamic shared memory.
+// The density pass's dynamic shared memory (plan() sizes it).
 struct DSmem {
+    unsigned char* feat;      // at its start, so that a slot's offset fits a queue entry: per pair of slots 16
+                              // bytes {x2, y2, z2, -}, fp16 cell coordinates from the region's centre; the
+                              // pair after the last one that fits is far from everything
     float4* sp;               // staged particles: x, y, z, rho_old
     int* s_gidx;              // global index of a staged slot
     int* s_off;               // region cell -> first slot (R + 1)
-    int* s_start;             // region cell -> first global index (R)
-    unsigned short* s_list;   // drain queue, DLIST x T (reuses s_start after staging)
+    unsigned short* s_list;   // drain queue, dlist x T: 8 x slot
     int* s_warp;
     int* s_work;              // work items {ox, oy, oz, ts, te}: the root, then two per split level
 };
@@ -352,11 +370,10 @@ __device__ __forceinline__ void density_region(const Phys& P, const DArgs& A, co
     float4* sp = M.sp;
     int* s_gidx = M.s_gidx;
     int* s_off = M.s_off;
-    int* s_start = M.s_start;
     unsigned short* s_list = M.s_list;
 
     // ---- stage the region: counts, scan (row-major by region cell), copy
-    const int total = region_offsets<BX, BY, BZ, H>(P, A.range, ox, oy, oz, s_off, s_start, s_gidx, C.cap, M.s_warp);
+    const int total = region_offsets<BX, BY, BZ, H>(P, A.range, ox, oy, oz, s_off, s_gidx, C.cap, M.s_warp);
     const bool staged = total <= C.cap;
     if constexpr (SPLITS > 0) {
         if (!staged) {
@@ -375,19 +392,28 @@ __device__ __forceinline__ void density_region(const Phys& P, const DArgs& A, co
             return;
         }
     }
+    const float cx = ((float)ox + 0.5f * BX) * P.dx, cy0 = ((float)oy + 0.5f * BY) * P.dy,
+                cz = ((float)oz + 0.5f * BZ) * P.dz;   // the region's centre
     if (staged) {
-        // slots strided over the block, copied global -> shared asynchronously:
-        // every slot of the thread in flight at once, no registers held (density
-        // 0.538 -> 0.527 ms at 2M against four register loads in flight)
-        for (int k = threadIdx.x; k < total; k += T) {
-            const unsigned d = (unsigned)__cvta_generic_to_shared(sp + k);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(A.pos + s_gidx[k]) : "memory");
+        // slots strided over the block, four loads in flight per thread
+        for (int k0 = threadIdx.x; k0 < total; k0 += 4 * T) {
+            float4 p[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k0 + u * T < total) p[u] = A.pos[s_gidx[k0 + u * T]];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (k0 + u * T < total) {
+                    const int k = k0 + u * T;
+                    sp[k] = p[u];
+                    __half* const f = reinterpret_cast<__half*>(M.feat + (k >> 1) * 16) + (k & 1);
+                    f[0] = feat_coord(p[u].x, cx, P.inv_dx);
+                    f[2] = feat_coord(p[u].y, cy0, P.inv_dy);
+                    f[4] = feat_coord(p[u].z, cz, P.inv_dz);
+                }
         }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
-
 
     // ---- targets, one warp-synchronous round of 32 targets at a time
     const int lane = threadIdx.x & 31;
@@ -414,69 +440,103 @@ __device__ __forceinline__ void density_region(const Phys& P, const DArgs& A, co
             if (active && !fast) A.defer[at + __popc(dm & ((1u << lane) - 1u))] = i;
         }
         NbrOut L{A.nbr, 0, P.N, i};
-        // the lanes' queues are the columns of the DLIST x T array (entry e of
-        // this lane at qlane[e T]); n counts the queued entries in units of T,
-        // so a push is one store and one add (density 0.5255 -> 0.5194 ms at 2M
-        // against indexing by the entry count)
+        // the lanes' queues are the columns of the dlist x T array, the next
+        // entry of this lane at shared address qat, so a push is one predicated
+        // store and one add
         unsigned short* const qlane = s_list + threadIdx.x;
-        const int qlim = (C.dlist - 4) * T;
-        int n = 0;
-        // all lanes drain their queues together, in lockstep
-#define ASPH_DRAIN()                                                                  \
-    do {                                                                              \
-        const int nmax_ = __reduce_max_sync(0xffffffffu, n);                          \
-        for (int q = 0; q < nmax_; q += T) {                                          \
-            if (q < n) {                                                              \
-                const int kq = qlane[q];                                              \
-                const float4 pj = sp[kq];                                             \
-                const float r2 = r2_pair(P, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z);      \
-                dsum_add(s, r2, pj.w, rr);                                            \
-                if (r2 >= 1e-12f) L.push(s_gidx[kq]);                                 \
-            }                                                                         \
-        }                                                                             \
-        n = 0;                                                                        \
+        const uint32_t q0 = (uint32_t)__cvta_generic_to_shared(qlane), qstep = 2u * (uint32_t)T;
+        uint32_t qat = q0;
+        // All lanes drain their queues together, in lockstep and without
+        // branches: an entry that fails the float test, and a lane whose queue has
+        // ended (it reads slot 0), adds zero to the sums and stores nothing.
+#define ASPH_DRAIN()                                                                      \
+    do {                                                                                  \
+        const int n_ = (int)(qat - q0) >> 1;                                              \
+        const int nmax_ = __reduce_max_sync(0xffffffffu, n_);                             \
+        for (int q_ = 0; q_ < nmax_; q_ += T) {                                           \
+            const uint32_t a_ = q_ < n_ ? qlane[q_] : 0u;                                 \
+            const float4 pj = *reinterpret_cast<const float4*>(spb + 2u * a_);            \
+            const int j_ = *reinterpret_cast<const int*>(gib + (a_ >> 1));                \
+            const float r2_ = r2_pair(P, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z);             \
+            const bool near_ = q_ < n_ && r2_ < 4.0f;                                     \
+            dsum_add_if(s, r2_, pj.w, rr, near_);                                         \
+            L.push_if(near_ && r2_ >= 1e-12f, j_);                                        \
+        }                                                                                 \
+        qat = q0;                                                                         \
     } while (0)
-        // flattened walk of the window rows in the staged region, branch
-        // free: every step advances a finished row (la = region cell of the
-        // row's first cell; rows step by RX, planes by RX * RY) and tests one
-        // candidate, with selects, so the lanes never diverge.  Lanes past
-        // their last row (la >= la_end) see empty rows.  The warp votes once
-        // per 4 steps, so queues drain at dlist - 4 (drains run on fuller queues
-        // than with a vote per 8 steps, which matters most in clustered states).
-        int la = 0, la_end = 0, cy = 0, k = 0, kend = 0;
-        if (fast) {
-            la = (zlo * G::RY + ly - STENCIL) * G::RX + lx - STENCIL;
-            la_end = la + (zhi - zlo + 1) * (G::RX * G::RY);
-            row_span(s_off, la, k, kend);
+        const unsigned char* const spb = reinterpret_cast<const unsigned char*>(sp);
+        const unsigned char* const gib = reinterpret_cast<const unsigned char*>(s_gidx);
+        // The walk: the window's rows one after another for the whole warp, two
+        // candidates a step, a pair of slots in fp16 (half2: seven
+        // operations for both against ten each in float).  The fp16 test only
+        // ever passes too many (FTHR); what passes is queued and takes the float test
+        // in the drain.  A lane whose row has ended tests what follows and takes none.
+        // Lanes of a warp have rows of much the same length (their windows
+        // overlap), so waiting for the longest one costs less than letting each
+        // lane run on into its next row, a dozen instructions more in every step.
+        // The next row's span is read one row ahead (a chain of latencies where few warps
+        // are left: 893 -> 876 us in the clustered state, 504 -> 466 even).
+        const __half2 xi2 = __half2half2(feat_coord(pi.x, cx, P.inv_dx));
+        const __half2 yi2 = __half2half2(feat_coord(pi.y, cy0, P.inv_dy));
+        const __half2 zi2 = __half2half2(feat_coord(pi.z, cz, P.inv_dz));
+        const uint32_t thr = h2_bits(__float2half2_rn(FTHR));
+        const int* ro = s_off + (zlo * G::RY + ly - STENCIL) * G::RX + lx - STENCIL;
+        const int planes = fast ? zhi - zlo + 1 : 0;
+        const int nplanes = __reduce_max_sync(0xffffffffu, planes);
+        int room = C.dlist;   // entries that certainly fit in every lane's queue
+        int kf = 0, ke = 0;   // the next row's slots, read one row ahead
+        if (planes > 0) {
+            kf = ro[0];
+            ke = ro[2 * STENCIL + 1];
         }
-        for (;;) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const bool adv = k >= kend;
-                int la2 = la + G::RX, cy2 = cy + 1;
-                const bool wrap = cy2 == 2 * STENCIL + 1;
-                la2 += wrap ? G::RX * G::RY - (2 * STENCIL + 1) * G::RX : 0;
-                cy2 = wrap ? 0 : cy2;
-                la = adv ? la2 : la;
-                cy = adv ? cy2 : cy;
-                if (adv) {   // predicated loads: only lanes that change rows read the offsets
-                    if (la < la_end) {
-                        k = s_off[la];
-                        kend = s_off[la + 2 * STENCIL + 1];
-                    } else {
-                        kend = k;
+        for (int jz = 0; jz < nplanes; ++jz) {
+            for (int jy = 0; jy <= 2 * STENCIL; ++jy) {
+                const int kfirst = kf * 8, kend = ke * 8;   // in 8-byte units of the features
+                ro += G::RX;
+                if (jy == 2 * STENCIL) ro += G::RX * G::RY - (2 * STENCIL + 1) * G::RX;
+                kf = ke = 0;
+                if (jz + (jy == 2 * STENCIL ? 1 : 0) < planes) {
+                    kf = ro[0];
+                    ke = ro[2 * STENCIL + 1];
+                }
+                int k = kfirst & ~15;
+                while (__any_sync(0xffffffffu, k < kend)) {
+                    const uint4 f = *reinterpret_cast<const uint4*>(M.feat + k);
+                    __half2 d = __hsub2(h2_of(f.x), xi2);
+                    __half2 r2 = __hmul2(d, d);
+                    d = __hsub2(h2_of(f.y), yi2);
+                    r2 = __hfma2(d, d, r2);
+                    d = __hsub2(h2_of(f.z), zi2);
+                    r2 = __hfma2(d, d, r2);
+                    asm volatile("{\n"
+                                 "  .reg .pred c, p, q;\n"
+                                 "  .reg .b16 e, o;\n"
+                                 "  setp.lt.s32 c, %3, %6;\n"
+                                 "  setp.le.and.f16x2 p|q, %1, %2, c;\n"
+                                 "  setp.ge.and.s32 p, %3, %4, p;\n"
+                                 "  setp.lt.and.s32 q, %5, %6, q;\n"
+                                 "  cvt.u16.u32 e, %3;\n"
+                                 "  cvt.u16.u32 o, %5;\n"
+                                 "  @p st.shared.u16 [%0], e;\n"
+                                 "  @p add.u32 %0, %0, %7;\n"
+                                 "  @q st.shared.u16 [%0], o;\n"
+                                 "  @q add.u32 %0, %0, %7;\n"
+                                 "}\n"
+                                 : "+r"(qat)
+                                 : "r"(h2_bits(r2)), "r"(thr), "r"(k), "r"(kfirst), "r"(k + 8), "r"(kend),
+                                   "r"(qstep)
+                                 : "memory");
+                    k += 16;
+                    room -= 2;
+                    if (room < 2) {   // as far as the steps tell: take the real room, drain when there is little
+                        room = C.dlist - (int)__umulhi(__reduce_max_sync(0xffffffffu, qat - q0), C.qinv);
+                        if (room < 4) {
+                            ASPH_DRAIN();
+                            room = C.dlist;
+                        }
                     }
                 }
-                const bool valid = k < kend;
-                const float4 pj = sp[valid ? k : 0];
-                if (valid && r2_pair(P, pi.x, pi.y, pi.z, pj.x, pj.y, pj.z) < 4.0f) {
-                    qlane[n] = (unsigned short)k;
-                    n += T;
-                }
-                k += valid ? 1 : 0;
             }
-            if (__any_sync(0xffffffffu, n > qlim)) ASPH_DRAIN();
-            if (__all_sync(0xffffffffu, la >= la_end)) break;
         }
         ASPH_DRAIN();
 #undef ASPH_DRAIN
@@ -494,20 +554,22 @@ __global__ __maxnreg__(DENSITY_REGS) void k_density_brick(const __grid_constant_
                                                        PairCfg C) {
     using G = BrickGeom<BX, BY, BZ, H>;
     extern __shared__ __align__(16) unsigned char smem[];
-    const int T = blockDim.x;
     __shared__ int s_warp[32];
     __shared__ int s_work[5 * (1 + 2 * DENSITY_SPLITS)];
     __shared__ int s_run;
     DSmem M;
-    M.sp = reinterpret_cast<float4*>(smem);
+    M.feat = smem;
+    M.sp = reinterpret_cast<float4*>(smem + (size_t)C.cap * 8 + 16);
     M.s_gidx = reinterpret_cast<int*>(M.sp + C.cap);
     M.s_off = M.s_gidx + C.cap;
-    M.s_start = M.s_off + (G::R + 1);
-    M.s_list = reinterpret_cast<unsigned short*>(M.s_start);
+    M.s_list = reinterpret_cast<unsigned short*>(M.s_off + (G::R + 1));
     M.s_warp = s_warp;
     M.s_work = s_work;
-    (void)T;
-    if (threadIdx.x == 0) s_run = A.ctl->aborted ? 0 : 1;   // one decision per block (barriers follow)
+    if (threadIdx.x == 0) {
+        s_run = A.ctl->aborted ? 0 : 1;   // one decision per block (barriers follow)
+        const uint32_t f = h2_bits(__float2half2_rn(1e4f));
+        *reinterpret_cast<uint4*>(M.feat + C.cap * 8) = make_uint4(f, f, f, f);
+    }
     __syncthreads();
     if (!s_run) return;
     const int b = blockIdx.x;
@@ -825,13 +887,22 @@ struct Shape {
 constexpr Shape SHAPES[] = {{8, 8, 8}, {8, 8, 4}, {8, 4, 4}, {4, 4, 4}};
 constexpr int MAX_STAGE = 4096;      // staged particles per brick at most
 constexpr double STAGE_MARGIN = 1.35;
+// Staging capacity that no launch goes below, over the expected count.  1.15 is
+// 1 % faster on an even lattice (465 against 470 us at 2M) and 1.35 leaves a
+// block fewer per SM there (487), but clustered bricks split more often with
+// less (830 us at 1.2, 876 at 1.15).
+constexpr double STAGE_NEED = 1.2;
 
 int region_cells(const Shape& s, int h) { return (s.bx + 2 * h) * (s.by + 2 * h) * (s.bz + 2 * h); }
 
-// Staged halo: with a sort every step the targets are in (or next to) the
-// cells of their brick, and the stencil alone is staged; slower cadences
-// stage one more cell of drift.  Targets outside either go to the deferred pass.
-int halo_for(const Phys& P) { return P.sort_every == 1 ? STENCIL : MAX_HALO; }
+// Staged halo: with a sort every step, or the displacement-gated sort (at
+// most 0.3 cells of drift along each axis), few targets have left their brick, and the
+// stencil alone is staged; slower cadences stage one more cell of drift.
+// Targets outside either go to the deferred pass, where one costs two to three
+// times as much as in its brick; under the gated sort they are at most 4 % along an axis
+// (0.3 of one layer in eight), 0.2 % in the runs measured, against 1.6 times the
+// cells to stage.
+int halo_for(const Phys& P) { return P.sort_every <= 1 ? STENCIL : MAX_HALO; }
 
 // Largest brick whose region fits the grid without wrapping onto itself
 // and whose expected staged count (with a margin) fits the cap.
@@ -841,11 +912,7 @@ bool fits(const Phys& P, int k) {
     return region_cells(s, MAX_HALO) * ((double)P.N / (double)P.ncell) * STAGE_MARGIN <= MAX_STAGE;
 }
 
-int pick_shape(const Phys& P) {
-    for (int k = 0; k < 4; ++k)
-        if (fits(P, k)) return k;
-    return -1;
-}
+int pick_shape(const Phys& P);
 
 int shape_in_use(const Phys& P, const Bufs& B) {
     if (B.force_global) return -1;
@@ -855,6 +922,7 @@ int shape_in_use(const Phys& P, const Bufs& B) {
 struct Launch {
     PairCfg C;
     int threads;
+    int blocks;   // resident per SM
     size_t smem;
 };
 
@@ -884,19 +952,19 @@ Launch plan(const Phys& P, const Shape& s, int h) {
     const int R = region_cells(s, h);
     // about one thread per expected target (the lattice keeps brick counts
     // close to the mean), in whole warps, 64..512
-    int t = (int)(s.bx * s.by * s.bz * ppc * 1.04 + 31) / 32 * 32;
-    L.threads = t < 64 ? 64 : (t > 512 ? 512 : t);
-    // s_start (R ints) while staging; the drain queue after
+    int groups = (int)(s.bx * s.by * s.bz * ppc * 1.04 + 31) / 32;
+    const int rounds = (groups + 15) / 16;
+    groups = (groups + rounds - 1) / rounds;
+    L.threads = 32 * (groups < 2 ? 2 : groups);
     auto smem_for = [&](size_t cap, int dlist) {
-        const size_t queue = (size_t)dlist * L.threads * 2, start = (size_t)4 * R;
-        return cap * 16 + cap * 4 + (size_t)4 * (R + 1) + ((queue > start ? queue : start) + 15) / 16 * 16;
+        return cap * (8 + 16 + 4) + 16 + (size_t)4 * (R + 1) + (size_t)dlist * L.threads * 2;
     };
     // staging capacity: at least the expected region count times STAGE_MARGIN;
     // the most resident blocks the registers allow come first, then the
     // deepest drain queue (fuller drains) that still fits them, then all the
     // shared memory left for staging, so that clustered bricks overflow less
     // often (an overflowing brick is split into halves)
-    int need = (int)(R * ppc * STAGE_MARGIN) + 64;
+    int need = (int)(R * ppc * STAGE_NEED) + 64;
     need = (need + 63) & ~63;
     need = need > MAX_STAGE ? MAX_STAGE : need;
     int per_sm, reserved;
@@ -904,6 +972,7 @@ Launch plan(const Phys& P, const Shape& s, int h) {
     const int by_regs = 65536 / (DENSITY_REGS * L.threads);
     int cap = need, dlist = 16;
     bool found = false;
+    L.blocks = 1;
     for (int b = by_regs < 8 ? by_regs : 8; b >= 1 && !found; --b) {
         const size_t budget = (size_t)(per_sm / b - reserved - 512);   // 512: the kernel's static arrays
         for (int d = DLIST; d >= 16 && !found; d -= 2) {
@@ -912,13 +981,35 @@ Launch plan(const Phys& P, const Shape& s, int h) {
             while (c > need && smem_for(c, d) > budget) c -= 64;
             cap = c;
             dlist = d;
+            L.blocks = b;
             found = true;
         }
     }
     L.C.cap = cap;
     L.C.dlist = dlist;
+    L.C.qinv = (uint32_t)((0x100000000ull + 2 * L.threads - 1) / (2 * L.threads));
     L.smem = smem_for(cap, dlist);
     return L;
+}
+
+// The largest brick (the smallest share of halo) whose blocks fill the GPU:
+// at least SHAPE_WARPS warps resident per SM, and at least four blocks for every
+// SM.  Staged slots and queues, not registers, limit the blocks of a large
+// brick in dense states: at one particle per cell 8 x 8 x 8 cells leave 18 warps per SM
+// and 8 x 8 x 4 leave 36 (density 473 against 433 us at 2M), at 0.6 both leave 40 (466
+// against 569 us); and 112 bricks of 32,768 particles take 88 us where 637 smaller
+// ones take 49.  It does not depend on the sort cadence, so the spans that one
+// step's gather wrote serve every other step of the context.
+constexpr int SHAPE_WARPS = 26;
+int pick_shape(const Phys& P) {
+    int k = 0;
+    while (k < 4 && !fits(P, k)) ++k;
+    if (k == 4) return -1;
+    for (; k < 3; ++k) {
+        const Launch L = plan(P, SHAPES[k], STENCIL);
+        if (L.blocks * (L.threads / 32) >= SHAPE_WARPS && L.C.nbricks >= 4 * 152) break;
+    }
+    return k;
 }
 
 // Blocks of the deferred pass: 4 per SM (32 warps), each warp looping over the queue.
