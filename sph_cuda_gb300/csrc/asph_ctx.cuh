@@ -39,6 +39,7 @@ struct asph_ctx {
     void* h_dump = nullptr;
     cudaEvent_t dump_ev = nullptr;
     bool dump_pending = false;
+    int* h_status = nullptr;    // pinned: the control block's words from `aborted` to `error`
     std::vector<void*> allocs;
 
     template <class T>
@@ -53,6 +54,7 @@ struct asph_ctx {
     }
     ~asph_ctx() {
         if (h_dump) cudaFreeHost(h_dump);
+        if (h_status) cudaFreeHost(h_status);
         if (dump_ev) cudaEventDestroy(dump_ev);
         for (auto& g : gexec)
             if (g) cudaGraphExecDestroy(g);
