@@ -57,6 +57,7 @@ struct Part {
     size_t bytes;
 };
 constexpr int NPARTS = 12;
+static_assert(NPARTS + 1 <= COPY_PARTS, "the parts and the control block go in one launch");
 
 int parts(asph_ctx* c, const asph_snapshot* s, Part out[NPARTS]) {
     const Bufs& B = c->B;
@@ -117,9 +118,12 @@ extern "C" int asph_snapshot_save(asph_ctx* c, asph_snapshot* s) {
     if (!same_shape(c, s)) return fail(ASPH_ERR_ARG, "snapshot was made for another particle count or grid");
     if (!c->initialised) return fail(ASPH_ERR_STATE, "snapshot before init/set_state");
     Part p[NPARTS];
+    CopyPart q[NPARTS + 1];
     const int n = parts(c, s, p);
-    for (int k = 0; k < n; ++k) CKR(cudaMemcpyAsync(p[k].snap, p[k].dev, p[k].bytes, cudaMemcpyDeviceToDevice, c->stream));
-    CKR(cudaMemcpyAsync(s->ctl, c->B.ctl, sizeof(DevCtl), cudaMemcpyDeviceToDevice, c->stream));
+    for (int k = 0; k < n; ++k) q[k] = CopyPart{p[k].dev, p[k].snap, p[k].bytes};
+    q[n] = CopyPart{c->B.ctl, s->ctl, sizeof(DevCtl)};
+    launch_copy_parts(q, n + 1, c->stream);
+    CKR(cudaGetLastError());
     return ASPH_OK;
 }
 
@@ -127,10 +131,13 @@ extern "C" int asph_snapshot_restore(asph_ctx* c, const asph_snapshot* s) {
     if (!c || !s) return fail(ASPH_ERR_ARG, "NULL argument");
     if (!same_shape(c, s)) return fail(ASPH_ERR_ARG, "snapshot was made for another particle count or grid");
     Part p[NPARTS];
+    CopyPart q[NPARTS + 1];
     const int n = parts(c, s, p);
-    for (int k = 0; k < n; ++k) CKR(cudaMemcpyAsync(p[k].dev, p[k].snap, p[k].bytes, cudaMemcpyDeviceToDevice, c->stream));
+    for (int k = 0; k < n; ++k) q[k] = CopyPart{p[k].snap, p[k].dev, p[k].bytes};
     // the radix look-back epoch keeps growing (status words of later sorts carry larger epochs)
-    CKR(cudaMemcpyAsync(c->B.ctl, s->ctl, offsetof(DevCtl, epoch), cudaMemcpyDeviceToDevice, c->stream));
+    q[n] = CopyPart{s->ctl, c->B.ctl, offsetof(DevCtl, epoch)};
+    launch_copy_parts(q, n + 1, c->stream);
+    CKR(cudaGetLastError());
     c->initialised = true;
     c->lists_valid = false;
     c->spans_valid = false;   // the restored sorted keys' brick spans are rebuilt before the next pass

@@ -163,6 +163,14 @@ AuditConst audit_constants(const AsphParams& p);
 void launch_audit(const Phys& P, const AuditConst& A, const Bufs& B, double* partial, int nblk, double* out,
                   cudaStream_t s);
 void launch_surf_flags(const Phys& P, const Bufs& B, uint8_t* flags, cudaStream_t s);
+// Copies of a snapshot, all in one launch: parts of any size, 16-byte aligned.
+constexpr int COPY_PARTS = 13;
+struct CopyPart {
+    const void* src;
+    void* dst;
+    size_t bytes;
+};
+void launch_copy_parts(const CopyPart* parts, int n, cudaStream_t s);
 void launch_coarse(const Phys& P, const Bufs& B, float* out, int sx, int sy, int sz, int cx, int cy,
                    int cz, float4* coldiag, cudaStream_t s);
 

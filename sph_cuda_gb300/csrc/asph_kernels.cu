@@ -358,8 +358,57 @@ __global__ void k_coldiag(const __grid_constant__ Phys P, const int2* __restrict
 }
 
 // ---------------------------------------------------------------------------
+// Snapshot copies: one launch for all parts.  Thirteen copies queued one by one cost
+// a small state about 2 us each on the host and on the stream; a block takes 16 KB
+// of one part, four 16-byte loads in flight per thread.
+// ---------------------------------------------------------------------------
+constexpr size_t COPY_TILE = (size_t)TPB * 4 * 16;
+struct CopyArgs {
+    const char* src[COPY_PARTS];
+    char* dst[COPY_PARTS];
+    size_t bytes[COPY_PARTS];
+    unsigned tile0[COPY_PARTS + 1];   // first block of each part
+};
+__global__ __launch_bounds__(TPB) void k_copy_parts(const __grid_constant__ CopyArgs A) {
+    int p = 0;
+    while (blockIdx.x >= A.tile0[p + 1]) ++p;
+    const size_t at = (size_t)(blockIdx.x - A.tile0[p]) * COPY_TILE, n = A.bytes[p] - at;
+    const char* src = A.src[p] + at;
+    char* dst = A.dst[p] + at;
+    uint4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const size_t o = ((size_t)u * TPB + threadIdx.x) * 16;
+        if (o + 16 <= n) v[u] = *reinterpret_cast<const uint4*>(src + o);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const size_t o = ((size_t)u * TPB + threadIdx.x) * 16;
+        if (o + 16 <= n) *reinterpret_cast<uint4*>(dst + o) = v[u];
+    }
+    // the last bytes of a part that are no whole 16
+    const size_t whole = n < COPY_TILE ? n & ~(size_t)15 : COPY_TILE;
+    if (n < COPY_TILE && whole + threadIdx.x < n) dst[whole + threadIdx.x] = src[whole + threadIdx.x];
+}
+
+// ---------------------------------------------------------------------------
 // launch functions
 // ---------------------------------------------------------------------------
+void launch_copy_parts(const CopyPart* parts, int n, cudaStream_t s) {
+    CopyArgs A{};
+    unsigned tiles = 0;
+    for (int k = 0; k < COPY_PARTS; ++k) {
+        A.tile0[k] = tiles;
+        if (k >= n) continue;
+        A.src[k] = (const char*)parts[k].src;
+        A.dst[k] = (char*)parts[k].dst;
+        A.bytes[k] = parts[k].bytes;
+        tiles += (unsigned)((parts[k].bytes + COPY_TILE - 1) / COPY_TILE);
+    }
+    A.tile0[COPY_PARTS] = tiles;
+    if (tiles) k_copy_parts<<<tiles, TPB, 0, s>>>(A);
+}
+
 static inline int blocks_for(int n) { return n <= 0 ? 1 : (n + TPB - 1) / TPB; }
 
 void launch_init(const Phys& P, const Bufs& B, const float* bub, int nbub, int init_mode, int lat_nx, int lat_ny,
