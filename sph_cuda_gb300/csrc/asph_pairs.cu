@@ -292,21 +292,40 @@ struct DArgs {
     DevCtl* ctl;
 };
 
+// First index of a sorted array whose value is not below `key`, by a whole
+// warp: 32 probes a round, so five dependent loads for 2M keys against 21.
+__device__ __forceinline__ int lower_bound_warp(const uint32_t* __restrict__ a, int n, uint32_t key) {
+    const int lane = threadIdx.x & 31;
+    int lo = 0;
+    for (;;) {
+        const int step = (n - lo + 31) / 32;   // probes at lo, lo + step, ...
+        const long long at = lo + (long long)lane * step;
+        const int below = __popc(__ballot_sync(0xffffffffu, at < n && __ldg(&a[at < n ? at : 0]) < key));
+        if (step <= 1) return lo + below;
+        if (below == 0) return lo;
+        const long long end = lo + (long long)below * step;   // the first probe not below, or past the end
+        lo += (below - 1) * step + 1;
+        n = end < n ? (int)end : n;
+        if (lo >= n) return lo;
+    }
+}
+
 // Every brick's span of targets in the sorted order: the brick is a
-// Morton-aligned key range, found by binary search in the sorted keys (one
-// thread per brick).  The gather writes the same spans when a sort runs; this
+// Morton-aligned key range, found by search in the sorted keys (a warp for each
+// end of a span).  The gather writes the same spans when a sort runs; this
 // kernel serves sorted keys that the gather did not see (a restored state,
-// another brick shape).
+// another brick shape): 13 -> 4 us at 475k particles against a thread per
+// brick and a binary search.
 template <int BX, int BY, int BZ>
 __global__ void k_brick_spans(const __grid_constant__ Phys P, const uint32_t* __restrict__ skeys, int2* spans,
                               PairCfg C) {
     using G = BrickGeom<BX, BY, BZ, STENCIL>;
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, b = w >> 1, upper = w & 1;
     if (b >= C.nbricks) return;
     const int bxi = b % C.nbx, byi = (b / C.nbx) % C.nby, bzi = b / (C.nbx * C.nby);
     const uint32_t base = morton3((uint32_t)(bxi * BX), (uint32_t)(byi * BY), (uint32_t)(bzi * BZ));
-    spans[base >> G::LOG2K] =
-        make_int2(lower_bound_u32(skeys, P.N, base), lower_bound_u32(skeys, P.N, base + (uint32_t)G::KEYS));
+    const int at = lower_bound_warp(skeys, P.N, base + (upper ? (uint32_t)G::KEYS : 0u));
+    if ((threadIdx.x & 31) == 0) reinterpret_cast<int*>(spans + (base >> G::LOG2K))[upper] = at;
 }
 
 __device__ __forceinline__ DSum density_target_global(const Phys& P, const DArgs& A, int i, float4 pi, FF rr) {
@@ -1061,7 +1080,7 @@ void launch_brick_spans(const Phys& P, const Bufs& B, cudaStream_t s) {
     if (k < 0) return;
     const Shape& sh = SHAPES[k];
     const Launch L = plan(P, sh, MAX_HALO);
-    const int blocks = (L.C.nbricks + 255) / 256;
+    const int blocks = (L.C.nbricks + 3) / 4;   // eight warps a block, two a brick
     switch (k) {
         case 0: k_brick_spans<8, 8, 8><<<blocks, 256, 0, s>>>(P, B.skeys, B.spans, L.C); break;
         case 1: k_brick_spans<8, 8, 4><<<blocks, 256, 0, s>>>(P, B.skeys, B.spans, L.C); break;
@@ -1105,6 +1124,15 @@ void launch_density(const Phys& P, const Bufs& B, cudaStream_t s) {
 }
 
 int momentum_tpt(const Bufs& B) { return B.m_tpt > 0 ? B.m_tpt : M_TPT; }
+// The default takes one target per thread where two would leave the GPU short of
+// threads (152 SMs x 1,024 resident): the lists of a thread's targets are
+// walked one after the other, and with idle SMs that is only latency.  Momentum
+// with one / two: 15.4 / 20.5 us at 16k, 17.4 / 20.5 at 65k, 22.5 / 32.8 at 32k and one
+// per cell, 47.1 / 51.2 at 262k; 59.9 / 59.0 at 475k and 217 / 211 at 2M.
+static int launch_tpt(const Phys& P, const Bufs& B) {
+    if (B.m_tpt > 0) return B.m_tpt;
+    return P.N <= 2 * 152 * 1024 ? 1 : M_TPT;
+}
 
 void launch_momentum(const Phys& P, const Bufs& B, int mode, int use_lists, cudaStream_t s) {
     MArgs A;
@@ -1128,7 +1156,7 @@ void launch_momentum(const Phys& P, const Bufs& B, int mode, int use_lists, cuda
     A.rain_out = B.rain[1 - B.rc];
     A.precip = B.precip;
     A.ctl = B.ctl;
-    const int tpt = momentum_tpt(B);
+    const int tpt = launch_tpt(P, B);
     A.part_blocks = blocks_for(P.N, M_TPB * tpt);
     const int rain_blocks = (mode & M_RAIN) ? blocks_for(P.ncell, M_TPB * M_RAIN_CELLS) : 0;
     A.rain_blocks = rain_blocks;
