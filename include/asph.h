@@ -387,7 +387,7 @@ int asph_set_viscosity(asph_ctx* ctx, float alpha, float beta);
  * the sort of asph_sort_build.  The sort runs over whole 8-bit digits, bits
  * [0, 8*ceil(key_bits/8)): keys must be below 2^key_bits (Morton keys of a
  * grid are) for that to be the sort over bits [0, key_bits).  Scratch lives
- * in a static device array sized for ASPH_NOALLOC_MAX_KEYS keys (about 5 MB,
+ * in a static device array sized for ASPH_NOALLOC_MAX_KEYS keys (about 7 MB,
  * held by every GPU that loads the library until exit); larger n returns
  * ASPH_ERR_ARG.  All calls share that array: calls that overlap on the GPU
  * race and must be serialised by the caller.  The outputs must not alias

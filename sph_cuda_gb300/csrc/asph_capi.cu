@@ -343,7 +343,7 @@ extern "C" int asph_create(const AsphParams* p, void* stream, asph_ctx** out) {
     }
     const size_t N = (size_t)P.N, C = (size_t)P.ncell;
     B.npasses = (P.key_bits + 7) / 8;
-    B.ntiles = (int)((N + SORT_TILE - 1) / SORT_TILE);
+    B.ntiles = sort_tiles(P.N);
     cudaError_t e = cudaSuccess;
 #define AL(ptr, bytes) \
     if (e == cudaSuccess) e = c->alloc(&(ptr), (bytes))

@@ -34,17 +34,11 @@
 
 namespace asph {
 
-// Kernels of asph_sort.cu, launched unchanged.
-__global__ void k_hist(const uint32_t* __restrict__ keys, int N, int npasses, DevCtl* __restrict__ ctl, int force,
-                       int lane);
-__global__ void k_radix_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
-                             uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, uint64_t* __restrict__ status,
-                             int N, int ntiles, int pass, DevCtl* __restrict__ ctl, int force, int lane);
-
 namespace {
 
 constexpr int NA_MAX_KEYS = ASPH_NOALLOC_MAX_KEYS;
-constexpr int NA_MAX_TILES = (NA_MAX_KEYS + SORT_TILE - 1) / SORT_TILE;
+constexpr int NA_MAX_TILES = 2 * 152;   // the smaller tiles are taken up to this many
+static_assert(sort_tiles(NA_MAX_KEYS) <= NA_MAX_TILES, "look-back words of the largest sort");
 constexpr size_t NA_CTL_BYTES = (sizeof(DevCtl) + 255) / 256 * 256;
 constexpr size_t NA_KEYS_OFF = NA_CTL_BYTES;
 constexpr size_t NA_VALS_OFF = NA_KEYS_OFF + (size_t)NA_MAX_KEYS * 4;
@@ -136,11 +130,8 @@ extern "C" int asph_sort_keys_noalloc(const uint32_t* keys, uint32_t* keys_sorte
     uint64_t* status = reinterpret_cast<uint64_t*>(base + NA_STATUS_OFF);
     cudaStream_t s = (cudaStream_t)stream;
     const int npasses = (key_bits + 7) / 8;
-    const int ntiles = (n + SORT_TILE - 1) / SORT_TILE;
     k_noalloc_prep<<<1, 256, 0, s>>>(ctl);
-    int hb = (n + TPB * 8 - 1) / (TPB * 8);
-    hb = hb > 152 * 8 ? 152 * 8 : hb;
-    k_hist<<<hb, SORT_TPB, 0, s>>>(keys, n, npasses, ctl, 1, 0);
+    launch_hist(keys, n, npasses, ctl, 1, 0, s);
     const uint32_t* ki = keys;
     const uint32_t* vi = nullptr;
     for (int p = 0; p < npasses; ++p) {
@@ -148,7 +139,7 @@ extern "C" int asph_sort_keys_noalloc(const uint32_t* keys, uint32_t* keys_sorte
         const bool to_out = ((npasses - 1 - p) % 2) == 0;
         uint32_t* ko = to_out ? keys_sorted : sk;
         uint32_t* vo = to_out ? perm : sv;
-        k_radix_pass<<<ntiles, SORT_TPB, 0, s>>>(ki, vi, ko, vo, status, n, ntiles, p, ctl, 1, 0);
+        launch_radix_pass(ki, vi, ko, vo, status, n, p, ctl, 1, 0, s);
         ki = ko;
         vi = vo;
     }

@@ -8,7 +8,7 @@
 //
 // Design (one "onesweep" pass per 8-bit digit):
 //  * one upfront histogram kernel counts the digits of every pass;
-//  * each pass kernel takes a tile of SORT_TILE keys (tile ids handed out by
+//  * each pass kernel takes a tile of keys (sort_tile(); tile ids handed out by
 //    an atomic counter so that a tile only ever waits on tiles that already
 //    started), ranks keys inside the tile with __match_any_sync warp
 //    ranking (stable: iteration order within a warp, warp order within the
@@ -28,6 +28,7 @@ namespace {
 constexpr uint64_t FLAG_AGG = 1ull << 30;
 constexpr uint64_t FLAG_PRE = 2ull << 30;
 constexpr uint64_t CNT_MASK = (1ull << 30) - 1;
+constexpr int LOOK_BACK = 4;   // predecessors read at a time
 
 // Gate of a sort launch (`force`): 0 the step's gating (the control
 // block's do_sort, nothing after an abort), 1 a forced full sort (granular
@@ -124,9 +125,15 @@ __global__ __launch_bounds__(SORT_TPB) void k_hist(const uint32_t* __restrict__ 
     __shared__ uint32_t h[MAX_PASSES][256];
     for (int i = threadIdx.x; i < MAX_PASSES * 256; i += blockDim.x) (&h[0][0])[i] = 0u;
     __syncthreads();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-        uint32_t k = keys[i];
-        for (int p = 0; p < npasses; ++p) atomicAdd(&h[p][(k >> (8 * p)) & 255u], 1u);
+    const int stride = gridDim.x * blockDim.x;
+    for (long long i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < N; i0 += 4ll * stride) {
+        uint32_t k[4];   // four keys in flight
+#pragma unroll
+        for (int u = 0; u < 4; ++u) k[u] = i0 + (long long)u * stride < N ? keys[i0 + (long long)u * stride] : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (i0 + (long long)u * stride < N)
+                for (int p = 0; p < npasses; ++p) atomicAdd(&h[p][(k[u] >> (8 * p)) & 255u], 1u);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < npasses * 256; i += blockDim.x) {
@@ -135,6 +142,7 @@ __global__ __launch_bounds__(SORT_TPB) void k_hist(const uint32_t* __restrict__ 
     }
 }
 
+template <int ITEMS>
 __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
     const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin, uint32_t* __restrict__ kout,
     uint32_t* __restrict__ vout, uint64_t* __restrict__ status, int N, int ntiles, int pass,
@@ -143,10 +151,10 @@ __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
     if (sort_lane) N = min(N, (int)ctl->inc_m);
     unsigned* const tile_ctr = sort_lane ? ctl->itile_ctr : ctl->tile_ctr;
     const unsigned* const ghist = sort_lane ? ctl->ihist[pass] : ctl->hist[pass];
-    constexpr int NW = SORT_TPB / 32;
+    constexpr int NW = SORT_TPB / 32, TILE = SORT_TPB * ITEMS;
     __shared__ uint32_t s_whist[NW][256];
-    __shared__ uint32_t s_keys[SORT_TILE];
-    __shared__ uint32_t s_vals[SORT_TILE];
+    __shared__ uint32_t s_keys[TILE];
+    __shared__ uint32_t s_vals[TILE];
     __shared__ uint32_t s_texcl[256];
     __shared__ uint32_t s_gbase[256];
     __shared__ uint32_t s_scan[NW];
@@ -157,16 +165,17 @@ __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
     for (int i = tid; i < NW * 256; i += SORT_TPB) (&s_whist[0][0])[i] = 0u;
     __syncthreads();
     const int tile = (int)s_tile;
+    const uint32_t gcount = ghist[tid];   // digit = thread; read here, needed after the look-back
     const int shift = 8 * pass;
-    const int base = tile * SORT_TILE;
+    const int base = tile * TILE;
     if (base >= N && tile > 0) return;   // lane 1 launches for its largest count
     const unsigned epoch = sort_lane ? ctl->iepoch : ctl->epoch;
 
-    uint32_t k[SORT_ITEMS], v[SORT_ITEMS], r[SORT_ITEMS];
-    uint32_t d[SORT_ITEMS];
+    uint32_t k[ITEMS], v[ITEMS], r[ITEMS];
+    uint32_t d[ITEMS];
 #pragma unroll
-    for (int it = 0; it < SORT_ITEMS; ++it) {
-        const int e = base + warp * 32 * SORT_ITEMS + it * 32 + lane;
+    for (int it = 0; it < ITEMS; ++it) {
+        const int e = base + warp * 32 * ITEMS + it * 32 + lane;
         const bool ok = e < N;
         k[it] = ok ? kin[e] : 0u;
         v[it] = ok ? (vin ? vin[e] : (uint32_t)e) : 0u;
@@ -175,7 +184,7 @@ __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
     // Stable rank inside the warp: iteration order, then lane order.
     const unsigned ltm = lanemask_lt();
 #pragma unroll
-    for (int it = 0; it < SORT_ITEMS; ++it) {
+    for (int it = 0; it < ITEMS; ++it) {
         const unsigned peers = __match_any_sync(0xffffffffu, d[it]);
         const int leader = __ffs(peers) - 1;
         uint32_t old = 0u;
@@ -207,20 +216,31 @@ __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
     } else {
         atomicExch((unsigned long long*)&st[(size_t)tile * 256 + dg],
                    (unsigned long long)(ep | FLAG_AGG | tile_cnt));
+        // The words of LOOK_BACK predecessors are read together, so a tile walks
+        // back several tiles per load latency.
         int t = tile - 1;
         unsigned spins = 0;
-        while (t >= 0) {
-            const uint64_t w = *(volatile const uint64_t*)&st[(size_t)t * 256 + dg];
-            if ((uint32_t)(w >> 32) != epoch || (w & (3ull << 30)) == 0) {
-                if (++spins > SPIN_LIMIT) {
-                    ctl->error = ASPH_ERR_TIMEOUT;
-                    break;
+        bool open = true;
+        while (open && t >= 0) {
+            uint64_t w[LOOK_BACK];
+#pragma unroll
+            for (int u = 0; u < LOOK_BACK; ++u)
+                w[u] = *(volatile const uint64_t*)&st[(size_t)max(t - u, 0) * 256 + dg];
+            int used = 0;
+#pragma unroll
+            for (int u = 0; u < LOOK_BACK; ++u) {
+                const bool ready = (uint32_t)(w[u] >> 32) == epoch && (w[u] & (3ull << 30)) != 0;
+                if (open && used == u && u <= t && ready) {   // in order, up to the first that is not there yet
+                    excl += (uint32_t)(w[u] & CNT_MASK);
+                    if (w[u] & FLAG_PRE) open = false;
+                    ++used;
                 }
-                continue;
             }
-            excl += (uint32_t)(w & CNT_MASK);
-            if (w & FLAG_PRE) break;
-            --t;
+            t -= used;
+            if (open && used == 0 && ++spins > SPIN_LIMIT) {
+                ctl->error = ASPH_ERR_TIMEOUT;
+                open = false;
+            }
         }
         atomicExch((unsigned long long*)&st[(size_t)tile * 256 + dg],
                    (unsigned long long)(ep | FLAG_PRE | (uint64_t)(excl + tile_cnt)));
@@ -229,7 +249,7 @@ __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
     // Global start of each digit (scan of the histogram) and the tile-local
     // start of each digit (scan of the tile counts).
     uint32_t tot;
-    const uint32_t gstart = block_excl_scan(ghist[dg], s_scan, &tot);
+    const uint32_t gstart = block_excl_scan(gcount, s_scan, &tot);
     const uint32_t texcl = block_excl_scan(tile_cnt, s_scan, &tot);
     s_texcl[dg] = texcl;
     s_gbase[dg] = gstart + excl;
@@ -237,7 +257,7 @@ __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
 
     // Local scatter into digit order, then coalesced runs to global.
 #pragma unroll
-    for (int it = 0; it < SORT_ITEMS; ++it) {
+    for (int it = 0; it < ITEMS; ++it) {
         if (d[it] < 256u) {
             const uint32_t lp = s_texcl[d[it]] + s_whist[warp][d[it]] + r[it];
             s_keys[lp] = k[it];
@@ -245,7 +265,7 @@ __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
         }
     }
     __syncthreads();
-    const int nvalid = max(0, min(SORT_TILE, N - base));
+    const int nvalid = max(0, min(TILE, N - base));
     for (int j = tid; j < nvalid; j += SORT_TPB) {
         const uint32_t key = s_keys[j];
         const uint32_t dd = (key >> shift) & 255u;
@@ -255,6 +275,19 @@ __global__ __launch_bounds__(SORT_TPB, 4) void k_radix_pass(
             vout[o] = s_vals[j];
         }
     }
+}
+
+void launch_hist(const uint32_t* keys, int n, int npasses, DevCtl* ctl, int force, int lane, cudaStream_t s) {
+    int blocks = (n + TPB * 8 - 1) / (TPB * 8);
+    blocks = blocks < 1 ? 1 : (blocks > 152 * 8 ? 152 * 8 : blocks);
+    k_hist<<<blocks, SORT_TPB, 0, s>>>(keys, n, npasses, ctl, force, lane);
+}
+
+void launch_radix_pass(const uint32_t* kin, const uint32_t* vin, uint32_t* kout, uint32_t* vout, uint64_t* status,
+                       int n, int pass, DevCtl* ctl, int force, int lane, cudaStream_t s) {
+    const int tiles = sort_tiles(n);
+    auto* k = sort_items(n) == 4 ? k_radix_pass<4> : (sort_items(n) == 8 ? k_radix_pass<8> : k_radix_pass<16>);
+    k<<<tiles, SORT_TPB, 0, s>>>(kin, vin, kout, vout, status, n, tiles, pass, ctl, force, lane);
 }
 
 // ---------------------------------------------------------------------------
@@ -448,7 +481,7 @@ __global__ __launch_bounds__(INC_TPB) void k_inc_merge(const uint32_t* __restric
 
 void sort_inc_sizes(int N, int* max_keys, int* tiles, int* blocks) {
     *max_keys = N / 8 > 0 ? N / 8 : 1;   // above this share of changed keys the full sort runs
-    *tiles = (*max_keys + SORT_TILE - 1) / SORT_TILE;
+    *tiles = sort_tiles(*max_keys);
     *blocks = (N + INC_CHUNK - 1) / INC_CHUNK;
 }
 
@@ -478,30 +511,24 @@ void launch_sort(const Phys& P, Bufs& B, int force, cudaStream_t s) {
         cudaEventRecord(B.ev_fork, s);
         cudaStreamWaitEvent(B.aux, B.ev_fork, 0);
     }
-    int hb = (P.N + TPB * 8 - 1) / (TPB * 8);
-    hb = hb > 152 * 8 ? 152 * 8 : hb;
-    k_hist<<<hb, SORT_TPB, 0, fs>>>(B.kin, P.N, B.npasses, B.ctl, force, 0);
+    launch_hist(B.kin, P.N, B.npasses, B.ctl, force, 0, fs);
     for (int p = 0; p < B.npasses; ++p) {
         const uint32_t* ki = p == 0 ? B.kin : B.kbuf[(p - 1) & 1];
         const uint32_t* vi = p == 0 ? nullptr : B.vbuf[(p - 1) & 1];
-        k_radix_pass<<<B.ntiles, SORT_TPB, 0, fs>>>(ki, vi, B.kbuf[p & 1], B.vbuf[p & 1], B.status, P.N,
-                                                    B.ntiles, p, B.ctl, force, 0);
+        launch_radix_pass(ki, vi, B.kbuf[p & 1], B.vbuf[p & 1], B.status, P.N, p, B.ctl, force, 0, fs);
     }
     if (fork) cudaEventRecord(B.ev_join, B.aux);
     if (inc) {
         k_inc_split<<<B.inc_blocks, INC_TPB, 0, s>>>(B.kin, B.skeys, P.N, B.inc_cnt, B.inc_u, B.inc_uk, B.inc_k[0],
                                                      B.inc_i[0] + 0, B.ctl, 0);
         // the changed keys: stable radix sort of (key, index), lane 1
-        int ib = (B.inc_max + TPB * 8 - 1) / (TPB * 8);
-        ib = ib < 1 ? 1 : (ib > 152 * 8 ? 152 * 8 : ib);
-        k_hist<<<ib, SORT_TPB, 0, s>>>(B.inc_k[0], B.inc_max, B.npasses, B.ctl, 0, 1);
+        launch_hist(B.inc_k[0], B.inc_max, B.npasses, B.ctl, 0, 1, s);
         const uint32_t* ki = B.inc_k[0];
         const uint32_t* vi = B.inc_i[0];
         for (int p = 0; p < B.npasses; ++p) {
             uint32_t* ko = B.inc_k[(p + 1) & 1];
             uint32_t* vo = B.inc_i[(p + 1) & 1];
-            k_radix_pass<<<B.inc_tiles, SORT_TPB, 0, s>>>(ki, vi, ko, vo, B.inc_status, B.inc_max, B.inc_tiles, p,
-                                                          B.ctl, 0, 1);
+            launch_radix_pass(ki, vi, ko, vo, B.inc_status, B.inc_max, p, B.ctl, 0, 1, s);
             ki = ko;
             vi = vo;
         }
@@ -536,9 +563,7 @@ void launch_sort_ahead(const Phys& P, Bufs& B, cudaStream_t s) {
     // skeys, ending in skeys_ahead, so the last applied sort stays intact
     cudaEventRecord(B.ev_fork, a);
     cudaStreamWaitEvent(B.aux, B.ev_fork, 0);
-    int hb = (P.N + TPB * 8 - 1) / (TPB * 8);
-    hb = hb > 152 * 8 ? 152 * 8 : hb;
-    k_hist<<<hb, SORT_TPB, 0, B.aux>>>(B.kin, P.N, B.npasses, B.ctl, GATE_AHEAD, 0);
+    launch_hist(B.kin, P.N, B.npasses, B.ctl, GATE_AHEAD, 0, B.aux);
     uint32_t* kscr = B.kbuf[B.skeys == B.kbuf[0] ? 1 : 0];
     uint32_t* vscr = B.vbuf[B.perm == B.vbuf[0] ? 1 : 0];
     const uint32_t* ki = B.kin;
@@ -547,8 +572,7 @@ void launch_sort_ahead(const Phys& P, Bufs& B, cudaStream_t s) {
         const bool last_parity = ((B.npasses - 1 - p) & 1) == 0;
         uint32_t* ko = last_parity ? B.skeys_ahead : kscr;
         uint32_t* vo = last_parity ? B.perm_ahead : vscr;
-        k_radix_pass<<<B.ntiles, SORT_TPB, 0, B.aux>>>(ki, vi, ko, vo, B.status, P.N, B.ntiles, p, B.ctl,
-                                                       GATE_AHEAD, 0);
+        launch_radix_pass(ki, vi, ko, vo, B.status, P.N, p, B.ctl, GATE_AHEAD, 0, B.aux);
         ki = ko;
         vi = vo;
     }
@@ -556,16 +580,13 @@ void launch_sort_ahead(const Phys& P, Bufs& B, cudaStream_t s) {
     // the incremental sort
     k_inc_split<<<B.inc_blocks, INC_TPB, 0, a>>>(B.kin, B.skeys, P.N, B.inc_cnt, B.inc_u, B.inc_uk, B.inc_k[0],
                                                  B.inc_i[0], B.ctl, GATE_AHEAD);
-    int ib = (B.inc_max + TPB * 8 - 1) / (TPB * 8);
-    ib = ib < 1 ? 1 : (ib > 152 * 8 ? 152 * 8 : ib);
-    k_hist<<<ib, SORT_TPB, 0, a>>>(B.inc_k[0], B.inc_max, B.npasses, B.ctl, GATE_AHEAD, 1);
+    launch_hist(B.inc_k[0], B.inc_max, B.npasses, B.ctl, GATE_AHEAD, 1, a);
     const uint32_t* ik = B.inc_k[0];
     const uint32_t* iv = B.inc_i[0];
     for (int p = 0; p < B.npasses; ++p) {
         uint32_t* ko = B.inc_k[(p + 1) & 1];
         uint32_t* vo = B.inc_i[(p + 1) & 1];
-        k_radix_pass<<<B.inc_tiles, SORT_TPB, 0, a>>>(ik, iv, ko, vo, B.inc_status, B.inc_max, B.inc_tiles, p,
-                                                      B.ctl, GATE_AHEAD, 1);
+        launch_radix_pass(ik, iv, ko, vo, B.inc_status, B.inc_max, p, B.ctl, GATE_AHEAD, 1, a);
         ik = ko;
         iv = vo;
     }
