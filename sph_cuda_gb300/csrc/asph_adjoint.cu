@@ -23,9 +23,8 @@
 //                       per-particle Jacobian by forward-mode dual numbers —
 //                       and the EOS
 //   R3 k_adj_dens_a/b   lagged Shepard density (pair gather)
-//   R2 k_adj_unperm     inverse of the sort's gather
-//   R1 k_adj_integrate  surface flux, drift with wrap/reflection, first kick
-//                       (order before the sort)
+//   R2, R1 k_adj_integrate  inverse of the sort's gather; surface flux, drift
+//                       with wrap/reflection, first kick (order before the sort)
 // Checkpoints: a device snapshot every `every` steps in the forward; the
 // backward restores each segment, recomputes it recording a per-step tape,
 // and reverses it.
@@ -216,8 +215,8 @@ struct StepTape {
     float4 *pos0, *vel0, *thq0, *acc0;   // step start, order before the sort
     uint8_t* surf0;                      // surface flags used by the flux
     uint32_t* perm;                      // the step's sort
-    float4 *pos1, *vel1, *thq1;          // after the gather: x1 (w = rho_old), v1, micro inputs
-    float2* rp;                          // rho, p'
+    float4 *pos1, *thq1;                 // after the gather: x1 (w = rho_old), micro inputs
+    float4 *ms0, *ms1;                   // x1, p' and v1, rho, as the density pass packs them for momentum
     float4* thq2;                        // micro outputs
     int *cnt, *lst;                      // neighbour lists, slot-major [NBR_CAP][N]
     float *rain0, *dep;                  // rain grid at the step start, deposits of the step
@@ -235,7 +234,6 @@ struct AdjBufs {
     float* lP;
     float2* lS;
     float *l_depc, *l_rain0;
-    float4 *px, *pv, *pq;
     double* ab;   // dJ/dalpha, dJ/dbeta
     int* err;
 };
@@ -265,8 +263,7 @@ __global__ void k_adj_rain(const Phys P, float dt, const float* __restrict__ rai
 __global__ void k_adj_mom_seed(const Phys P, float dt, StepTape T, AdjBufs A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
-    const float4 x1 = T.pos1[i], v1 = T.vel1[i], t2 = T.thq2[i], a = T.acc[i];
-    const float2 rp = T.rp[i];
+    const float4 x1 = T.ms0[i], v1 = T.ms1[i], t2 = T.thq2[i], a = T.acc[i];   // x1.w = p'
     const float dthdt = T.dthdt[i];
     const float4 ep = A.e_pos[i], ev = A.e_vel[i], eq = A.e_thq[i], ea = A.e_acc[i];
     const float z = x1.z, hdt = 0.5f * dt;
@@ -292,7 +289,7 @@ __global__ void k_adj_mom_seed(const Phys P, float dt, StepTape T, AdjBufs A) {
     const float I2 = fabsf(dthdt) < P.dthdt_cap ? 1.f : 0.f;
     const float ldth = I2 * ldthdt;
     const float pref = snd_eval(P.snd_p, P.snd_n, z).v();
-    const float pflm_raw = pref + rp.y;
+    const float pflm_raw = pref + x1.w;
     const float pflm = fmaxf(pflm_raw, 1.f);
     const float Pi = powf(pflm / P0, KAPPA);
     const float cpPi = CP * Pi;
@@ -326,98 +323,128 @@ __global__ void k_adj_mom_seed(const Phys P, float dt, StepTape T, AdjBufs A) {
 // R5b: momentum pair sums.  For the pair (i, j) in i's list, the thread of
 // i takes the derivative of i's own pair term (seeds of i) and of the term
 // i contributes to j's sum (seeds of j) with respect to i's variables.
-__global__ __launch_bounds__(ATPB, 4) void k_adj_mom_pairs(const Phys P, StepTape T, AdjBufs A) {
+// Bound by the latency of the neighbours' gathers: a neighbour is four 16-byte
+// records (the density pass's packed x, p' and v, rho, and the two seeds; five
+// loads from the state buffers before), and two neighbours' loads are in
+// flight before their arithmetic.
+struct AdjPairSum {
+    float gx, gy, gz, gvx, gvy, gvz, grho, gP, Vx, Vy, Vz, la, lb;
+};
+struct AdjPairTarget {
+    float4 x, v, sF, sV;   // x.w = p', v.w = rho
+    float rho, irho, I;    // clamped rho, 1 / rho, d rho / d v.w
+};
+__device__ __forceinline__ void adj_mom_pair(const Phys& P, const AdjPairTarget& t, const float4& xj, const float4& vj,
+                                             const float4& sFj, const float4& sVj, AdjPairSum& g) {
+    const float4 &xi = t.x, &vi = t.v, &sFi = t.sF, &sVi = t.sV;
+    const float rhoi = t.rho, iri = t.irho, Ii = t.I;
+    const float Mx = P.inv_dx * P.inv_dx, My = P.inv_dy * P.inv_dy, Mz = P.inv_dz * P.inv_dz;
+    // the pair geometry exactly as the forward pass forms it (msum_add)
+    const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+    const float dxt = rx * P.inv_dx, dyt = ry * P.inv_dy, dzt = rz * P.inv_dz;
+    const float r2t = __fmaf_rn(dxt, dxt, __fmaf_rn(dyt, dyt, dzt * dzt));
+    if (r2t < 1e-12f) return;
+    const float rs = rsqrt_normal(r2t);
+    const float qq = r2t * rs;
+    const float t2 = 2.f - qq;
+    // W'(q)/q and its q-derivative (both branches as in the forward)
+    const float kq = qq < 1.f ? SIGMA_W * __fmaf_rn(2.25f, qq, -3.f) : (-0.75f * SIGMA_W) * (t2 * t2) * rs;
+    const float kpq = qq < 1.f ? (2.25f * SIGMA_W) * rs : (0.75f * SIGMA_W) * t2 * (qq + 2.f) * (rs * rs * rs);
+    const float Mrx = Mx * rx, Mry = My * ry, Mrz = Mz * rz;   // M r
+    const float gxx = kq * Mrx, gyy = kq * Mry, gzz = kq * Mrz;   // grad_i W
+    const float rhoj = fmaxf(vj.w, 1e-3f), irj = rcp_normal(rhoj);
+    const float dp = (xj.w - xi.w) * (iri * irj);   // dp_ij ; dp_ji = -dp
+    const float ux = vi.x - vj.x, uy = vi.y - vj.y, uz = vi.z - vj.z;
+    const float sdot = __fmaf_rn(ux, rx, __fmaf_rn(uy, ry, uz * rz));
+    float mu = 0.f, hd = 0.f, m2 = 0.f, Phi = 0.f, dPhi = 0.f;
+    const float rbar = 0.5f * (rhoi + rhoj), irb = rcp_normal(rbar), ir2 = irb * irb;
+    const bool vis = sdot < 0.f;
+    if (vis) {
+        const float iden = rcp_normal(__fmaf_rn(rx, rx, __fmaf_rn(ry, ry, rz * rz)) + P.eta2);
+        hd = P.h_av * iden;
+        mu = hd * sdot;
+        m2 = 2.f * mu * iden;
+        Phi = mu * __fmaf_rn(P.beta, mu, -P.alpha * P.cs);
+        dPhi = __fmaf_rn(2.f * P.beta, mu, -P.alpha * P.cs);
+    }
+    const float visc_ij = Phi * (irj * ir2);   // in i's sum
+    const float visc_ji = Phi * (iri * ir2);   // in j's sum
+    g.Vx = __fmaf_rn(-visc_ij, gxx, g.Vx); g.Vy = __fmaf_rn(-visc_ij, gyy, g.Vy); g.Vz = __fmaf_rn(-visc_ij, gzz, g.Vz);
+    // ---- (a) i's own term, seeds of i; (b) the term of j's sum in which i is
+    // the neighbour, seeds of j (g_ji = -g_ij, dp_ji = -dp).  Both give
+    // dc/dx_i = +-(kq M c + kpq (r.Mc) M r) with c = dc/dg.
+    const float Aa = __fmaf_rn(sFi.x, gxx, __fmaf_rn(sFi.y, gyy, sFi.z * gzz));
+    const float Ba = __fmaf_rn(sVi.x, gxx, __fmaf_rn(sVi.y, gyy, sVi.z * gzz));
+    const float Ab = -__fmaf_rn(sFj.x, gxx, __fmaf_rn(sFj.y, gyy, sFj.z * gzz));
+    const float Bb = -__fmaf_rn(sVj.x, gxx, __fmaf_rn(sVj.y, gyy, sVj.z * gzz));
+    const float bra = dp + visc_ij, brb = visc_ji - dp;
+    // c_a - c_b (the x_i derivative of (b) enters with a minus sign)
+    const float cx = -bra * sFi.x - visc_ij * sVi.x + brb * sFj.x + visc_ji * sVj.x;
+    const float cy = -bra * sFi.y - visc_ij * sVi.y + brb * sFj.y + visc_ji * sVj.y;
+    const float cz = -bra * sFi.z - visc_ij * sVi.z + brb * sFj.z + visc_ji * sVj.z;
+    const float rMc = __fmaf_rn(Mrx, cx, __fmaf_rn(Mry, cy, Mrz * cz));
+    g.gx += __fmaf_rn(kq * Mx, cx, kpq * rMc * Mrx);
+    g.gy += __fmaf_rn(kq * My, cy, kpq * rMc * Mry);
+    g.gz += __fmaf_rn(kq * Mz, cz, kpq * rMc * Mrz);
+    g.gP += (Aa - Ab) * (iri * irj);
+    g.grho += Ii * (Aa - Ab) * dp * iri;
+    if (vis) {
+        const float Psa = -(Aa + Ba), Psb = -(Ab + Bb);
+        const float lmu = dPhi * ir2 * (Psa * irj + Psb * iri);
+        g.gvx = __fmaf_rn(lmu * hd, rx, g.gvx);
+        g.gvy = __fmaf_rn(lmu * hd, ry, g.gvy);
+        g.gvz = __fmaf_rn(lmu * hd, rz, g.gvz);
+        g.gx = __fmaf_rn(lmu, __fmaf_rn(hd, ux, -m2 * rx), g.gx);
+        g.gy = __fmaf_rn(lmu, __fmaf_rn(hd, uy, -m2 * ry), g.gy);
+        g.gz = __fmaf_rn(lmu, __fmaf_rn(hd, uz, -m2 * rz), g.gz);
+        // visc_ij = Phi / (rho_j rbar^2), visc_ji = Phi / (rho_i rbar^2), rbar = (rho_i + rho_j)/2
+        g.grho += Ii * (Psa * (-visc_ij * irb) + Psb * (-visc_ji) * (iri + irb));
+        const float wa = Psa * (irj * ir2);
+        g.la = __fmaf_rn(wa, -P.cs * mu, g.la);
+        g.lb = __fmaf_rn(wa, mu * mu, g.lb);
+    }
+}
+
+constexpr int PAIR_TPB = 128;   // a block ends with its longest list
+
+__global__ __launch_bounds__(PAIR_TPB, 5) void k_adj_mom_pairs(const __grid_constant__ Phys P,
+                                                               const __grid_constant__ StepTape T,
+                                                               const __grid_constant__ AdjBufs A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     float la = 0.f, lb = 0.f;
     if (i < P.N) {
-        const float4 xi = T.pos1[i], vi = T.vel1[i], sFi = A.sF[i], sVi = A.sV[i];
-        const float2 ri = T.rp[i];
-        const float rhoi = fmaxf(ri.x, 1e-3f), iri = __fdividef(1.f, rhoi);
-        const float Ii = ri.x > 1e-3f ? 1.f : 0.f;
+        AdjPairTarget t;
+        t.x = T.ms0[i]; t.v = T.ms1[i]; t.sF = A.sF[i]; t.sV = A.sV[i];
+        t.rho = fmaxf(t.v.w, 1e-3f);
+        t.irho = rcp_normal(t.rho);
+        t.I = t.v.w > 1e-3f ? 1.f : 0.f;
         const int cnt = T.cnt[i];
         if (cnt < 0) atomicExch(A.err, 1);   // list overflow: the adjoint needs every pair
-        float gx = 0.f, gy = 0.f, gz = 0.f, gvx = 0.f, gvy = 0.f, gvz = 0.f, grho = 0.f, gP = 0.f;
-        float Vx = 0.f, Vy = 0.f, Vz = 0.f;
-        const float Mx = P.inv_dx * P.inv_dx, My = P.inv_dy * P.inv_dy, Mz = P.inv_dz * P.inv_dz;
-        for (int q = 0; q < cnt; ++q) {
-            const int j = T.lst[(size_t)q * P.N + i];
-            const float4 xj = T.pos1[j], vj = T.vel1[j], sFj = A.sF[j], sVj = A.sV[j];
-            const float2 rj = T.rp[j];
-            // the pair geometry exactly as the forward pass forms it (msum_add)
-            const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-            const float dxt = rx * P.inv_dx, dyt = ry * P.inv_dy, dzt = rz * P.inv_dz;
-            const float r2t = __fmaf_rn(dxt, dxt, __fmaf_rn(dyt, dyt, dzt * dzt));
-            if (r2t < 1e-12f) continue;
-            const float rs = rsqrtf(r2t);
-            const float qq = r2t * rs;
-            const float t2 = 2.f - qq;
-            // W'(q)/q and its q-derivative (both branches as in the forward)
-            const float kq = qq < 1.f ? SIGMA_W * __fmaf_rn(2.25f, qq, -3.f) : (-0.75f * SIGMA_W) * (t2 * t2) * rs;
-            const float kpq = qq < 1.f ? (2.25f * SIGMA_W) * rs : (0.75f * SIGMA_W) * t2 * (qq + 2.f) * (rs * rs * rs);
-            const float Mrx = Mx * rx, Mry = My * ry, Mrz = Mz * rz;   // M r
-            const float gxx = kq * Mrx, gyy = kq * Mry, gzz = kq * Mrz;   // grad_i W
-            const float rhoj = fmaxf(rj.x, 1e-3f), irj = __fdividef(1.f, rhoj);
-            const float dp = (rj.y - ri.y) * (iri * irj);   // dp_ij ; dp_ji = -dp
-            const float ux = vi.x - vj.x, uy = vi.y - vj.y, uz = vi.z - vj.z;
-            const float sdot = __fmaf_rn(ux, rx, __fmaf_rn(uy, ry, uz * rz));
-            float mu = 0.f, hd = 0.f, m2 = 0.f, Phi = 0.f, dPhi = 0.f;
-            const float rbar = 0.5f * (rhoi + rhoj), irb = __fdividef(1.f, rbar), ir2 = irb * irb;
-            const bool vis = sdot < 0.f;
-            if (vis) {
-                const float iden = __fdividef(1.f, __fmaf_rn(rx, rx, __fmaf_rn(ry, ry, rz * rz)) + P.eta2);
-                hd = P.h_av * iden;
-                mu = hd * sdot;
-                m2 = 2.f * mu * iden;
-                Phi = mu * __fmaf_rn(P.beta, mu, -P.alpha * P.cs);
-                dPhi = __fmaf_rn(2.f * P.beta, mu, -P.alpha * P.cs);
-            }
-            const float visc_ij = Phi * (irj * ir2);   // in i's sum
-            const float visc_ji = Phi * (iri * ir2);   // in j's sum
-            Vx = __fmaf_rn(-visc_ij, gxx, Vx); Vy = __fmaf_rn(-visc_ij, gyy, Vy); Vz = __fmaf_rn(-visc_ij, gzz, Vz);
-            // ---- (a) i's own term, seeds of i; (b) the term of j's sum in which i is
-            // the neighbour, seeds of j (g_ji = -g_ij, dp_ji = -dp).  Both give
-            // dc/dx_i = +-(kq M c + kpq (r.Mc) M r) with c = dc/dg.
-            const float Aa = __fmaf_rn(sFi.x, gxx, __fmaf_rn(sFi.y, gyy, sFi.z * gzz));
-            const float Ba = __fmaf_rn(sVi.x, gxx, __fmaf_rn(sVi.y, gyy, sVi.z * gzz));
-            const float Ab = -__fmaf_rn(sFj.x, gxx, __fmaf_rn(sFj.y, gyy, sFj.z * gzz));
-            const float Bb = -__fmaf_rn(sVj.x, gxx, __fmaf_rn(sVj.y, gyy, sVj.z * gzz));
-            const float bra = dp + visc_ij, brb = visc_ji - dp;
-            // c_a - c_b (the x_i derivative of (b) enters with a minus sign)
-            const float cx = -bra * sFi.x - visc_ij * sVi.x + brb * sFj.x + visc_ji * sVj.x;
-            const float cy = -bra * sFi.y - visc_ij * sVi.y + brb * sFj.y + visc_ji * sVj.y;
-            const float cz = -bra * sFi.z - visc_ij * sVi.z + brb * sFj.z + visc_ji * sVj.z;
-            const float rMc = __fmaf_rn(Mrx, cx, __fmaf_rn(Mry, cy, Mrz * cz));
-            gx += __fmaf_rn(kq * Mx, cx, kpq * rMc * Mrx);
-            gy += __fmaf_rn(kq * My, cy, kpq * rMc * Mry);
-            gz += __fmaf_rn(kq * Mz, cz, kpq * rMc * Mrz);
-            gP += (Aa - Ab) * (iri * irj);
-            grho += Ii * (Aa - Ab) * dp * iri;
-            if (vis) {
-                const float Psa = -(Aa + Ba), Psb = -(Ab + Bb);
-                const float lmu = dPhi * ir2 * (Psa * irj + Psb * iri);
-                gvx = __fmaf_rn(lmu * hd, rx, gvx); gvy = __fmaf_rn(lmu * hd, ry, gvy); gvz = __fmaf_rn(lmu * hd, rz, gvz);
-                gx = __fmaf_rn(lmu, __fmaf_rn(hd, ux, -m2 * rx), gx);
-                gy = __fmaf_rn(lmu, __fmaf_rn(hd, uy, -m2 * ry), gy);
-                gz = __fmaf_rn(lmu, __fmaf_rn(hd, uz, -m2 * rz), gz);
-                // visc_ij = Phi / (rho_j rbar^2), visc_ji = Phi / (rho_i rbar^2), rbar = (rho_i + rho_j)/2
-                grho += Ii * (Psa * (-visc_ij * irb) + Psb * (-visc_ji) * (iri + irb));
-                const float wa = Psa * (irj * ir2);
-                la = __fmaf_rn(wa, -P.cs * mu, la);
-                lb = __fmaf_rn(wa, mu * mu, lb);
-            }
+        AdjPairSum g{};
+        const int* lp = T.lst + i;
+        const size_t N = (size_t)P.N;
+        for (int q = 0; q < cnt; q += 2, lp += 2 * N) {
+            const bool two = q + 1 < cnt;
+            const int j0 = lp[0], j1 = two ? lp[N] : j0;
+            const float4 x0 = T.ms0[j0], v0 = T.ms1[j0], f0 = A.sF[j0], w0 = A.sV[j0];
+            const float4 x1 = T.ms0[j1], v1 = T.ms1[j1], f1 = A.sF[j1], w1 = A.sV[j1];
+            adj_mom_pair(P, t, x0, v0, f0, w0, g);
+            if (two) adj_mom_pair(P, t, x1, v1, f1, w1, g);
         }
+        la = g.la;
+        lb = g.lb;
         // heating: d dth / d v1 = -Vm / (cp Pi)
-        const float ldth = sFi.w, cpPi = sVi.w;
-        gvx += -P.mm * Vx / cpPi * ldth;
-        gvy += -P.mm * Vy / cpPi * ldth;
-        gvz += -P.mm * Vz / cpPi * ldth;
+        const float ldth = t.sF.w, cpPi = t.sV.w;
+        g.gvx += -P.mm * g.Vx / cpPi * ldth;
+        g.gvy += -P.mm * g.Vy / cpPi * ldth;
+        g.gvz += -P.mm * g.Vz / cpPi * ldth;
         float4 lx = A.lx[i];
-        lx.x += gx; lx.y += gy; lx.z += gz; lx.w += grho;
+        lx.x += g.gx; lx.y += g.gy; lx.z += g.gz; lx.w += g.grho;
         A.lx[i] = lx;
         float4 lv = A.lv[i];
-        lv.x += gvx; lv.y += gvy; lv.z += gvz;
+        lv.x += g.gvx; lv.y += g.gvy; lv.z += g.gvz;
         A.lv[i] = lv;
-        A.lP[i] += gP;
+        A.lP[i] += g.gP;
     }
     // dJ/dalpha, dJ/dbeta: warp sums, one double atomic per warp
 #pragma unroll
@@ -435,8 +462,8 @@ __global__ __launch_bounds__(ATPB, 4) void k_adj_mom_pairs(const Phys P, StepTap
 __global__ void k_adj_micro(const Phys P, float dt, StepTape T, AdjBufs A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
-    const float4 x1 = T.pos1[i], t1 = T.thq1[i];
-    const float2 rp = T.rp[i];
+    const float4 x1 = T.ms0[i], t1 = T.thq1[i];
+    const float2 rp = make_float2(T.ms1[i].w, x1.w);
     const float z = x1.z;
     const int cid = cell_of(P, x1.x, x1.y, z);
     const float pref = snd_eval(P.snd_p, P.snd_n, z).v();
@@ -481,22 +508,35 @@ __global__ void k_adj_micro(const Phys P, float dt, StepTape T, AdjBufs A) {
 }
 
 // R3a: density sums of the target and the adjoint of rho = clamp(S1/S2).
-__global__ void k_adj_dens_a(const Phys P, StepTape T, AdjBufs A) {
+// Four neighbours' loads in flight, as in R3b.
+__global__ __launch_bounds__(PAIR_TPB, 8) void k_adj_dens_a(const __grid_constant__ Phys P,
+                                                            const __grid_constant__ StepTape T,
+                                                            const __grid_constant__ AdjBufs A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const float4 xi = T.pos1[i];
     float S1 = w3(0.f), S2 = __fdividef(w3(0.f), fmaxf(xi.w, 1e-3f));   // self pair
     const int cnt = T.cnt[i];
-    for (int q = 0; q < cnt; ++q) {
-        const int j = T.lst[(size_t)q * P.N + i];
-        const float4 xj = T.pos1[j];
-        const float r2t = r2_pair(P, xi.x, xi.y, xi.z, xj.x, xj.y, xj.z);   // the density pass's own r^2
-        if (r2t >= 4.f || r2t < 1e-12f) continue;
-        const float qq = r2t * rsqrtf(r2t), t = 2.f - qq;
-        const float W = qq < 1.f ? SIGMA_W * __fmaf_rn(qq * qq, __fmaf_rn(0.75f, qq, -1.5f), 1.f)
-                                 : (0.25f * SIGMA_W) * (t * t * t);
-        S1 += W;
-        S2 += __fdividef(W, fmaxf(xj.w, 1e-3f));
+    const int* lp = T.lst + i;
+    const size_t N = (size_t)P.N;
+    for (int q = 0; q < cnt; q += 4, lp += 4 * N) {
+        int j[4];
+        float4 x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) j[u] = q + u < cnt ? lp[u * N] : i;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = T.pos1[j[u]];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float4 xj = x[u];
+            const float r2t = r2_pair(P, xi.x, xi.y, xi.z, xj.x, xj.y, xj.z);   // the density pass's own r^2
+            if (r2t >= 4.f || r2t < 1e-12f) continue;   // (the padding is the target itself)
+            const float qq = r2t * rsqrtf(r2t), t = 2.f - qq;
+            const float W = qq < 1.f ? SIGMA_W * __fmaf_rn(qq * qq, __fmaf_rn(0.75f, qq, -1.5f), 1.f)
+                                     : (0.25f * SIGMA_W) * (t * t * t);
+            S1 += W;
+            S2 += __fdividef(W, fmaxf(xj.w, 1e-3f));
+        }
     }
     float4 lx = A.lx[i];
     const float lrho = lx.w;
@@ -517,34 +557,51 @@ __global__ void k_adj_dens_a(const Phys P, StepTape T, AdjBufs A) {
     A.lS[i] = make_float2(lS1, lS2);
 }
 
-// R3b: density pairs: positions and the lagged densities rho_old.
-__global__ __launch_bounds__(ATPB) void k_adj_dens_b(const Phys P, StepTape T, AdjBufs A) {
+// R3b: density pairs: positions and the lagged densities rho_old.  Four
+// neighbours' loads in flight, as in the forward momentum pass.
+__global__ __launch_bounds__(PAIR_TPB, 8) void k_adj_dens_b(const __grid_constant__ Phys P,
+                                                            const __grid_constant__ StepTape T,
+                                                            const __grid_constant__ AdjBufs A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
     const float4 xi = T.pos1[i];
     const float2 lSi = A.lS[i];
-    const float roi = fmaxf(xi.w, 1e-3f), iroi = __fdividef(1.f, roi);
+    const float roi = fmaxf(xi.w, 1e-3f), iroi = rcp_normal(roi);
     const float Mx = P.inv_dx * P.inv_dx, My = P.inv_dy * P.inv_dy, Mz = P.inv_dz * P.inv_dz;
     float gx = 0.f, gy = 0.f, gz = 0.f;
     float lro = lSi.y * (-w3(0.f) * iroi * iroi);   // self pair in S2_i
     const int cnt = T.cnt[i];
-    for (int q = 0; q < cnt; ++q) {
-        const int j = T.lst[(size_t)q * P.N + i];
-        const float4 xj = T.pos1[j];
-        const float2 lSj = A.lS[j];
-        const float r2t = r2_pair(P, xi.x, xi.y, xi.z, xj.x, xj.y, xj.z);   // the density pass's own r^2
-        if (r2t >= 4.f || r2t < 1e-12f) continue;
-        const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
-        const float rs = rsqrtf(r2t), qq = r2t * rs, t = 2.f - qq;
-        const float W = qq < 1.f ? SIGMA_W * __fmaf_rn(qq * qq, __fmaf_rn(0.75f, qq, -1.5f), 1.f)
-                                 : (0.25f * SIGMA_W) * (t * t * t);
-        const float kq = qq < 1.f ? SIGMA_W * __fmaf_rn(2.25f, qq, -3.f) : (-0.75f * SIGMA_W) * (t * t) * rs;
-        const float iroj = __fdividef(1.f, fmaxf(xj.w, 1e-3f));
-        const float c = (lSi.x + lSj.x) + lSi.y * iroj + lSj.y * iroi;
-        gx += c * kq * Mx * rx;
-        gy += c * kq * My * ry;
-        gz += c * kq * Mz * rz;
-        lro += lSj.y * (-W * iroi * iroi);   // i is a neighbour in S2_j
+    const int* lp = T.lst + i;
+    const size_t N = (size_t)P.N;
+    for (int q = 0; q < cnt; q += 4, lp += 4 * N) {
+        int j[4];
+        float4 x[4];
+        float2 l[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) j[u] = q + u < cnt ? lp[u * N] : i;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            x[u] = T.pos1[j[u]];
+            l[u] = A.lS[j[u]];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float4 xj = x[u];
+            const float2 lSj = l[u];
+            const float r2t = r2_pair(P, xi.x, xi.y, xi.z, xj.x, xj.y, xj.z);   // the density pass's own r^2
+            if (r2t >= 4.f || r2t < 1e-12f) continue;   // (the padding is the target itself)
+            const float rx = xi.x - xj.x, ry = xi.y - xj.y, rz = xi.z - xj.z;
+            const float rs = rsqrt_normal(r2t), qq = r2t * rs, t = 2.f - qq;
+            const float W = qq < 1.f ? SIGMA_W * __fmaf_rn(qq * qq, __fmaf_rn(0.75f, qq, -1.5f), 1.f)
+                                     : (0.25f * SIGMA_W) * (t * t * t);
+            const float kq = qq < 1.f ? SIGMA_W * __fmaf_rn(2.25f, qq, -3.f) : (-0.75f * SIGMA_W) * (t * t) * rs;
+            const float iroj = rcp_normal(fmaxf(xj.w, 1e-3f));
+            const float c = (lSi.x + lSj.x) + lSi.y * iroj + lSj.y * iroi;
+            gx += c * kq * Mx * rx;
+            gy += c * kq * My * ry;
+            gz += c * kq * Mz * rz;
+            lro += lSj.y * (-W * iroi * iroi);   // i is a neighbour in S2_j
+        }
     }
     if (!(xi.w > 1e-3f)) lro = 0.f;
     float4 lx = A.lx[i];
@@ -552,23 +609,15 @@ __global__ __launch_bounds__(ATPB) void k_adj_dens_b(const Phys P, StepTape T, A
     A.lx[i] = lx;
 }
 
-// R2: inverse of the gather new[k] = old[perm[k]].
-__global__ void k_adj_unperm(const Phys P, const uint32_t* __restrict__ perm, AdjBufs A) {
+// R2, R1: inverse of the sort's gather new[k] = old[perm[k]], then the
+// surface flux, drift and first half kick of particle perm[k] in the order
+// before the sort; writes the adjoint of the previous step's end state.
+__global__ void k_adj_integrate(const Phys P, float dt, float Ts, float qs_sfc, StepTape T, AdjBufs A) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= P.N) return;
-    const uint32_t i = perm[k];
-    A.px[i] = A.lx[k];
-    A.pv[i] = A.lv[k];
-    A.pq[i] = A.lq[k];
-}
-
-// R1: surface flux, drift, first half kick (order before the sort); writes
-// the adjoint of the previous step's end state.
-__global__ void k_adj_integrate(const Phys P, float dt, float Ts, float qs_sfc, StepTape T, AdjBufs A) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= P.N) return;
+    const uint32_t i = T.perm[k];
     const float4 x0 = T.pos0[i], v0 = T.vel0[i], t0 = T.thq0[i], a0 = T.acc0[i];
-    const float4 lx = A.px[i], lv = A.pv[i], lq = A.pq[i];
+    const float4 lx = A.lx[k], lv = A.lv[k], lq = A.lq[k];
     const float hdt = 0.5f * dt;
     const float vzp = v0.z + a0.z * hdt;
     const float zp = x0.z + (v0.z + a0.z * hdt) * dt;
@@ -602,6 +651,24 @@ __global__ void k_adj_integrate(const Phys P, float dt, float Ts, float qs_sfc, 
     A.e_vel[i] = make_float4(lvpx, lvpy, lvpz, 0.f);
     A.e_thq[i] = make_float4(lth0, lqv0, lq.z, 0.f);
     A.e_acc[i] = make_float4(hdt * lvpx, hdt * lvpy, hdt * lvpz, 0.f);
+}
+
+// The terminal adjoint from the caller's arrays as they are (any NULL: zero),
+// and the gradient of theta0 as one array.
+__global__ void k_adj_terminal(int N, const float* __restrict__ dqc, const float* __restrict__ dth,
+                               const float* __restrict__ dxyz, AdjBufs A) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= N) return;
+    const size_t n = (size_t)N;
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    A.e_thq[i] = make_float4(dth ? dth[i] : 0.f, 0.f, dqc ? dqc[i] : 0.f, 0.f);
+    A.e_pos[i] = dxyz ? make_float4(dxyz[i], dxyz[n + i], dxyz[2 * n + i], 0.f) : zero;
+    A.e_vel[i] = zero;
+    A.e_acc[i] = zero;
+}
+__global__ void k_adj_result(int N, AdjBufs A, float* __restrict__ dth0) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < N) dth0[i] = A.e_thq[i].x;
 }
 
 }  // namespace
@@ -672,10 +739,11 @@ int af_step(asph_adj* a, StepTape* t) {
     // the window runs without the source-term hook (its tendencies are not differentiated)
     float4* const src = B.src;
     B.src = nullptr;
-#define CP_(dst, src, bytes) CKR(cudaMemcpyAsync((dst), (src), (bytes), cudaMemcpyDeviceToDevice, s))
     if (t) {
-        CP_(t->pos0, B.pos[B.pc], N * 16); CP_(t->vel0, B.vel[B.vc], N * 16); CP_(t->thq0, B.thq[B.qc], N * 16);
-        CP_(t->acc0, B.acc, N * 16); CP_(t->surf0, B.surf, N); CP_(t->rain0, B.rain[B.rc], C * 4);
+        const CopyPart q[] = {{B.pos[B.pc], t->pos0, N * 16}, {B.vel[B.vc], t->vel0, N * 16},
+                              {B.thq[B.qc], t->thq0, N * 16}, {B.acc, t->acc0, N * 16},
+                              {B.surf, t->surf0, N},          {B.rain[B.rc], t->rain0, C * 4}};
+        launch_copy_parts(q, 6, s);
     }
     launch_gather(P, B, G_INTEGRATE, s);   // kick, drift, flux, keys (current order)
     B.pc ^= 1; B.vc ^= 1; B.qc ^= 1;
@@ -684,28 +752,30 @@ int af_step(asph_adj* a, StepTape* t) {
     launch_gather(P, B, G_SORTED | G_FORCE, s);   // reorder, cell table, surface flags
     B.pc ^= 1; B.vc ^= 1; B.qc ^= 1;
     if (t) {
-        CP_(t->perm, B.perm, N * 4);
-        CP_(t->pos1, B.pos[B.pc], N * 16); CP_(t->vel1, B.vel[B.vc], N * 16); CP_(t->thq1, B.thq[B.qc], N * 16);
+        const CopyPart q[] = {{B.perm, t->perm, N * 4}, {B.pos[B.pc], t->pos1, N * 16}, {B.thq[B.qc], t->thq1, N * 16}};
+        launch_copy_parts(q, 3, s);
     }
-    // a recorded step writes its neighbour lists straight into the tape
-    int* const nbr = B.nbr;
-    int* const nbr_cnt = B.nbr_cnt;
-    if (t) { B.nbr = t->lst; B.nbr_cnt = t->cnt; }
+    // a recorded step writes its neighbour lists and packed momentum sources
+    // straight into the tape
+    const Bufs own = B;
+    if (t) {
+        B.nbr = t->lst; B.nbr_cnt = t->cnt;
+        B.ms[0] = t->ms0; B.ms[1] = t->ms1;
+    }
     launch_density(P, B, s);
     if (t) {
-        CP_(t->rp, B.rp, N * 8); CP_(t->thq2, B.thq[B.qc], N * 16);
-        if (reads_rain(P)) CP_(t->dep, B.rain_delta, C * 4);
+        const CopyPart q[] = {{B.thq[B.qc], t->thq2, N * 16}};
+        launch_copy_parts(q, 1, s);
     }
     launch_momentum(P, B, M_INTEGRATE | M_RAIN | M_CFL, 1, s);
-    B.nbr = nbr;
-    B.nbr_cnt = nbr_cnt;
+    B = own;
     B.src = src;
     B.vc ^= 1; B.rc ^= 1;
     if (t) {
-        CP_(t->acc, B.acc, N * 16); CP_(t->dthdt, B.dthdt, N * 4);
+        const CopyPart q[] = {{B.acc, t->acc, N * 16}, {B.dthdt, t->dthdt, N * 4}, {B.rain_delta, t->dep, C * 4}};
+        launch_copy_parts(q, reads_rain(P) ? 3 : 2, s);
         c->lists_valid = false;   // the context's own lists are from an earlier step
     }
-#undef CP_
     CKR(cudaGetLastError());
     if (!t) c->lists_valid = true;
     return ASPH_OK;
@@ -769,14 +839,13 @@ void reverse_step(asph_adj* a, StepTape& t, cudaStream_t s) {
     k_adj_rain<<<blocks(P.ncell), ATPB, 0, s>>>(P, dt, t.rain0, t.dep, A.e_rain, A.l_rain0, A.l_depc,
                                                 reads_rain(P) ? 1 : 0);
     k_adj_mom_seed<<<blocks(P.N), ATPB, 0, s>>>(P, dt, t, A);
-    k_adj_mom_pairs<<<blocks(P.N), ATPB, 0, s>>>(P, t, A);
+    const int pair_blocks = (P.N + PAIR_TPB - 1) / PAIR_TPB;
+    k_adj_mom_pairs<<<pair_blocks, PAIR_TPB, 0, s>>>(P, t, A);
     k_adj_micro<<<blocks(P.N), ATPB, 0, s>>>(P, dt, t, A);
-    k_adj_dens_a<<<blocks(P.N), ATPB, 0, s>>>(P, t, A);
-    k_adj_dens_b<<<blocks(P.N), ATPB, 0, s>>>(P, t, A);
-    k_adj_unperm<<<blocks(P.N), ATPB, 0, s>>>(P, t.perm, A);
+    k_adj_dens_a<<<pair_blocks, PAIR_TPB, 0, s>>>(P, t, A);
+    k_adj_dens_b<<<pair_blocks, PAIR_TPB, 0, s>>>(P, t, A);
     k_adj_integrate<<<blocks(P.N), ATPB, 0, s>>>(P, dt, Ts, qs, t, A);
-    // the rain adjoint of the previous step's end
-    cudaMemcpyAsync(A.e_rain, A.l_rain0, (size_t)P.ncell * 4, cudaMemcpyDeviceToDevice, s);
+    std::swap(A.e_rain, A.l_rain0);   // the rain adjoint of the previous step's end
 }
 
 }  // namespace
@@ -802,7 +871,7 @@ extern "C" int asph_adj_create(asph_ctx* c, int nsteps, int every, asph_adj** ou
 #define AL(p, b) if (e == cudaSuccess) e = a->alloc(&(p), (b))
     for (auto& t : a->tape) {
         AL(t.pos0, N * 16); AL(t.vel0, N * 16); AL(t.thq0, N * 16); AL(t.acc0, N * 16); AL(t.surf0, N);
-        AL(t.perm, N * 4); AL(t.pos1, N * 16); AL(t.vel1, N * 16); AL(t.thq1, N * 16); AL(t.rp, N * 8);
+        AL(t.perm, N * 4); AL(t.pos1, N * 16); AL(t.ms0, N * 16); AL(t.ms1, N * 16); AL(t.thq1, N * 16);
         AL(t.thq2, N * 16); AL(t.cnt, N * 4); AL(t.lst, (size_t)NBR_CAP * N * 4); AL(t.rain0, C * 4);
         AL(t.dep, C * 4); AL(t.acc, N * 16); AL(t.dthdt, N * 4);
     }
@@ -810,7 +879,7 @@ extern "C" int asph_adj_create(asph_ctx* c, int nsteps, int every, asph_adj** ou
     AL(A.e_pos, N * 16); AL(A.e_vel, N * 16); AL(A.e_thq, N * 16); AL(A.e_acc, N * 16); AL(A.e_rain, C * 4);
     AL(A.sF, N * 16); AL(A.sV, N * 16); AL(A.lx, N * 16); AL(A.lv, N * 16); AL(A.lq, N * 16);
     AL(A.lP, N * 4); AL(A.lS, N * 8); AL(A.l_depc, C * 4); AL(A.l_rain0, C * 4);
-    AL(A.px, N * 16); AL(A.pv, N * 16); AL(A.pq, N * 16); AL(A.ab, 16); AL(A.err, 16);
+    AL(A.ab, 16); AL(A.err, 16);
 #undef AL
     if (!st && e != cudaSuccess)
         st = fail(e == cudaErrorMemoryAllocation ? ASPH_ERR_NOMEM : ASPH_ERR_CUDA, "adjoint allocation: %s",
@@ -867,24 +936,17 @@ extern "C" int asph_adj_backward(asph_adj* a, const float* dL_dqc, const float* 
     const size_t N = (size_t)P.N, C = (size_t)P.ncell;
     AdjBufs& A = a->A;
     int st = ASPH_OK;
-    // terminal adjoint: dL/dqc and dL/dtheta of the final state (its order)
-    std::vector<float> h(N * 4, 0.f);
-    for (size_t i = 0; i < N; ++i) {
-        h[4 * i + 0] = dL_dtheta ? dL_dtheta[i] : 0.f;
-        h[4 * i + 2] = dL_dqc ? dL_dqc[i] : 0.f;
-    }
-    CKR(cudaMemcpyAsync(A.e_thq, h.data(), N * 16, cudaMemcpyHostToDevice, s));
-    std::vector<float> hp(N * 4, 0.f);
-    if (dL_dxyz)
-        for (size_t i = 0; i < N; ++i) {
-            hp[4 * i + 0] = dL_dxyz[i];
-            hp[4 * i + 1] = dL_dxyz[N + i];
-            hp[4 * i + 2] = dL_dxyz[2 * N + i];
-        }
-    CKR(cudaMemcpyAsync(A.e_pos, hp.data(), N * 16, cudaMemcpyHostToDevice, s));
-    CKR(cudaStreamSynchronize(s));   // the host staging vectors go out of scope below
-    CKR(cudaMemsetAsync(A.e_vel, 0, N * 16, s));
-    CKR(cudaMemsetAsync(A.e_acc, 0, N * 16, s));
+    // terminal adjoint: dL/dqc and dL/dtheta of the final state (its order),
+    // copied as they are into buffers that the reverse fills later (packing them
+    // on the host took 1 ms of a 262k backward)
+    float* const up_qc = reinterpret_cast<float*>(A.sF);
+    float* const up_th = up_qc + N;
+    float* const up_xyz = reinterpret_cast<float*>(A.sV);
+    if (dL_dqc) CKR(cudaMemcpyAsync(up_qc, dL_dqc, N * 4, cudaMemcpyHostToDevice, s));
+    if (dL_dtheta) CKR(cudaMemcpyAsync(up_th, dL_dtheta, N * 4, cudaMemcpyHostToDevice, s));
+    if (dL_dxyz) CKR(cudaMemcpyAsync(up_xyz, dL_dxyz, N * 12, cudaMemcpyHostToDevice, s));
+    k_adj_terminal<<<blocks(P.N), ATPB, 0, s>>>(P.N, dL_dqc ? up_qc : nullptr, dL_dtheta ? up_th : nullptr,
+                                                dL_dxyz ? up_xyz : nullptr, A);
     CKR(cudaMemsetAsync(A.e_rain, 0, C * 4, s));
     CKR(cudaMemsetAsync(A.ab, 0, 16, s));
     CKR(cudaMemsetAsync(A.err, 0, 16, s));
@@ -903,10 +965,12 @@ extern "C" int asph_adj_backward(asph_adj* a, const float* dL_dqc, const float* 
     double ab[2];
     CKR(cudaMemcpyAsync(&err, A.err, sizeof(int), cudaMemcpyDeviceToHost, s));
     CKR(cudaMemcpyAsync(ab, A.ab, sizeof ab, cudaMemcpyDeviceToHost, s));
-    CKR(cudaMemcpyAsync(h.data(), A.e_thq, N * 16, cudaMemcpyDeviceToHost, s));
     CKR(cudaStreamSynchronize(s));
     if (err) return fail(ASPH_ERR_STATE, "a neighbour list overflowed inside the adjoint window");
-    for (size_t i = 0; i < N; ++i) dL_dtheta0[i] = h[4 * i];
+    float* const down = reinterpret_cast<float*>(A.sF);
+    k_adj_result<<<blocks(P.N), ATPB, 0, s>>>(P.N, A, down);
+    CKR(cudaMemcpyAsync(dL_dtheta0, down, N * 4, cudaMemcpyDeviceToHost, s));
+    CKR(cudaStreamSynchronize(s));
     if (dL_dalpha_beta) {
         dL_dalpha_beta[0] = ab[0];
         dL_dalpha_beta[1] = ab[1];

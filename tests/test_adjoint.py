@@ -216,3 +216,31 @@ def test_torch_autograd_function():
     assert _rel(th0.grad.numpy(), dth) < 1e-4
     assert abs(alpha.grad.item() - da) <= 1e-4 * abs(da)
     sim.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lat", [(13, 11, 17), (16, 16, 16)])
+def test_backward_is_linear_in_its_seeds(lat):
+    """The gradient of a sum of losses is the sum of their gradients, with any
+    of the three seed arrays absent, at particle counts that fill no block."""
+    from sph_cuda_gb300 import Asph
+    from sph_cuda_gb300.adjoint import AdjointWindow
+    from statebuild import random_state, small_config
+    p = small_config(lat=lat)
+    s = random_state(p, 41, "jitter")
+    sim = Asph(p)
+    sim.set_state(s)
+    sim.sort_build()
+    win = AdjointWindow(sim, 2, 1)
+    win.forward()
+    rng = np.random.default_rng(3)
+    n = p.n_particles
+    seeds = {"dL_dqc": rng.normal(size=n).astype(np.float32), "dL_dtheta": rng.normal(size=n).astype(np.float32),
+             "dL_dxyz": (1e-3 * rng.normal(size=3 * n)).astype(np.float32)}
+    parts = [win.backward(**{k: v})[0].astype(np.float64) for k, v in seeds.items()]
+    both = win.backward(**seeds)[0].astype(np.float64)
+    # float32 reverse sums of about 50 terms per particle and step: 1e-5 of the largest part
+    scale = max(np.abs(q).max() for q in parts)
+    assert np.abs(sum(parts) - both).max() < 1e-5 * scale
+    win.close()
+    sim.close()
