@@ -37,6 +37,7 @@ struct DevCtl {
     unsigned split_last;       // ... in the last density pass
     unsigned gmax[3];          // float bits of |u|,|v|,|w| maxima (atomicMax)
     unsigned epoch;            // radix look-back epoch
+    unsigned clamp_blocks;     // finished blocks of a velocity clamp (the last clears clamp_pending)
     unsigned hist[MAX_PASSES][256];
     unsigned tile_ctr[MAX_PASSES];
     // incremental sort (sort lane 1): keys that changed since the last sort

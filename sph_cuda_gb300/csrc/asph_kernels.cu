@@ -249,7 +249,10 @@ __global__ void k_cfl_ctl(const __grid_constant__ Phys P, DevCtl* __restrict__ c
 // Emergency clamp |v| <= 0.5 c_s when a CFL trip is pending
 // (asph_h100.cu:669-675, 1067-1068).
 __global__ void k_clamp(const __grid_constant__ Phys P, float4* __restrict__ vel, DevCtl* __restrict__ ctl) {
-    if (!ctl->clamp_pending) return;
+    __shared__ int s_pending;
+    if (threadIdx.x == 0) s_pending = ctl->clamp_pending;   // one decision per block
+    __syncthreads();
+    if (!s_pending) return;
     const float vmax = 0.5f * P.cs;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < P.N; i += gridDim.x * blockDim.x) {
         float4 v = vel[i];
@@ -260,8 +263,13 @@ __global__ void k_clamp(const __grid_constant__ Phys P, float4* __restrict__ vel
             vel[i] = v;
         }
     }
+    // every block has read the flag before the last one to finish clears it
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(&ctl->clamp_blocks, 1u) == gridDim.x - 1) {
+        ctl->clamp_blocks = 0u;
+        ctl->clamp_pending = 0;
+    }
 }
-__global__ void k_clamp_done(DevCtl* ctl) { ctl->clamp_pending = 0; }
 
 // ---------------------------------------------------------------------------
 // FP64 conservation audit (asph_h100.cu:650-668), deterministic two-stage.
@@ -456,8 +464,9 @@ void launch_cfl(const Phys& P, const Bufs& B, cudaStream_t s) {
 }
 
 void launch_clamp(const Phys& P, const Bufs& B, cudaStream_t s) {
-    k_clamp<<<152 * 4, TPB, 0, s>>>(P, B.vel[B.vc], B.ctl);
-    k_clamp_done<<<1, 1, 0, s>>>(B.ctl);
+    int blocks = blocks_for(P.N);
+    blocks = blocks > 152 * 4 ? 152 * 4 : blocks;
+    k_clamp<<<blocks, TPB, 0, s>>>(P, B.vel[B.vc], B.ctl);
 }
 
 void launch_audit(const Phys& P, const AuditConst& A, const Bufs& B, double* partial, int nblk, double* out,
