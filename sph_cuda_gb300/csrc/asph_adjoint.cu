@@ -216,7 +216,7 @@ struct StepTape {
     uint8_t* surf0;                      // surface flags used by the flux
     uint32_t* perm;                      // the step's sort
     float4 *pos1, *thq1;                 // after the gather: x1 (w = rho_old), micro inputs
-    float4 *ms0, *ms1;                   // x1, p' and v1, rho, as the density pass packs them for momentum
+    float4* ms;                          // x1, p' and v1, rho, as the density pass packs them for momentum
     float4* thq2;                        // micro outputs
     int *cnt, *lst;                      // neighbour lists, slot-major [NBR_CAP][N]
     float *rain0, *dep;                  // rain grid at the step start, deposits of the step
@@ -230,7 +230,8 @@ struct AdjBufs {
     float4 *e_pos, *e_vel, *e_thq, *e_acc;
     float* e_rain;
     // intermediates
-    float4 *sF, *sV, *lx, *lv, *lq;
+    float4* sFV;   // seeds of the momentum pair sums, 32 bytes a particle
+    float4 *lx, *lv, *lq;
     float* lP;
     float2* lS;
     float *l_depc, *l_rain0;
@@ -263,7 +264,9 @@ __global__ void k_adj_rain(const Phys P, float dt, const float* __restrict__ rai
 __global__ void k_adj_mom_seed(const Phys P, float dt, StepTape T, AdjBufs A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
-    const float4 x1 = T.ms0[i], v1 = T.ms1[i], t2 = T.thq2[i], a = T.acc[i];   // x1.w = p'
+    const float4 t2 = T.thq2[i], a = T.acc[i];
+    float4 x1, v1;   // x1.w = p'
+    ldg_record(T.ms, i, x1, v1);
     const float dthdt = T.dthdt[i];
     const float4 ep = A.e_pos[i], ev = A.e_vel[i], eq = A.e_thq[i], ea = A.e_acc[i];
     const float z = x1.z, hdt = 0.5f * dt;
@@ -310,8 +313,8 @@ __global__ void k_adj_mom_seed(const Phys P, float dt, StepTape T, AdjBufs A) {
     const float lqc2 = eq.z - GRAV * laz;
     lz += laz * (-GRAV * t2.x * fac * snd_slope(P.snd_thvr, P.snd_n, z) / (thvr * thvr));
     const float cv = -ldth / cpPi;
-    A.sF[i] = make_float4(P.mm * lax, P.mm * lay, P.mm * laz, ldth);
-    A.sV[i] = make_float4(P.mm * cv * v1.x, P.mm * cv * v1.y, P.mm * cv * v1.z, cpPi);
+    stg_record(A.sFV, i, make_float4(P.mm * lax, P.mm * lay, P.mm * laz, ldth),
+               make_float4(P.mm * cv * v1.x, P.mm * cv * v1.y, P.mm * cv * v1.z, cpPi));
     // the step's final positions are the drifted x1: their adjoint carries on;
     // w: dJ/drho of this step's density (the next step's rho_old)
     A.lx[i] = make_float4(ep.x, ep.y, ep.z + lz, ep.w);
@@ -323,8 +326,8 @@ __global__ void k_adj_mom_seed(const Phys P, float dt, StepTape T, AdjBufs A) {
 // R5b: momentum pair sums.  For the pair (i, j) in i's list, the thread of
 // i takes the derivative of i's own pair term (seeds of i) and of the term
 // i contributes to j's sum (seeds of j) with respect to i's variables.
-// Bound by the latency of the neighbours' gathers: a neighbour is four 16-byte
-// records (the density pass's packed x, p' and v, rho, and the two seeds; five
+// Bound by the latency of the neighbours' gathers: a neighbour is two 32-byte
+// records (the density pass's packed x, p', v, rho, and the two seeds; five
 // loads from the state buffers before), and two neighbours' loads are in
 // flight before their arithmetic.
 struct AdjPairSum {
@@ -414,7 +417,8 @@ __global__ __launch_bounds__(PAIR_TPB, 5) void k_adj_mom_pairs(const __grid_cons
     float la = 0.f, lb = 0.f;
     if (i < P.N) {
         AdjPairTarget t;
-        t.x = T.ms0[i]; t.v = T.ms1[i]; t.sF = A.sF[i]; t.sV = A.sV[i];
+        ldg_record(T.ms, i, t.x, t.v);
+        ldg_record(A.sFV, i, t.sF, t.sV);
         t.rho = fmaxf(t.v.w, 1e-3f);
         t.irho = rcp_normal(t.rho);
         t.I = t.v.w > 1e-3f ? 1.f : 0.f;
@@ -426,8 +430,11 @@ __global__ __launch_bounds__(PAIR_TPB, 5) void k_adj_mom_pairs(const __grid_cons
         for (int q = 0; q < cnt; q += 2, lp += 2 * N) {
             const bool two = q + 1 < cnt;
             const int j0 = lp[0], j1 = two ? lp[N] : j0;
-            const float4 x0 = T.ms0[j0], v0 = T.ms1[j0], f0 = A.sF[j0], w0 = A.sV[j0];
-            const float4 x1 = T.ms0[j1], v1 = T.ms1[j1], f1 = A.sF[j1], w1 = A.sV[j1];
+            float4 x0, v0, f0, w0, x1, v1, f1, w1;
+            ldg_record(T.ms, j0, x0, v0);
+            ldg_record(A.sFV, j0, f0, w0);
+            ldg_record(T.ms, j1, x1, v1);
+            ldg_record(A.sFV, j1, f1, w1);
             adj_mom_pair(P, t, x0, v0, f0, w0, g);
             if (two) adj_mom_pair(P, t, x1, v1, f1, w1, g);
         }
@@ -462,8 +469,10 @@ __global__ __launch_bounds__(PAIR_TPB, 5) void k_adj_mom_pairs(const __grid_cons
 __global__ void k_adj_micro(const Phys P, float dt, StepTape T, AdjBufs A) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.N) return;
-    const float4 x1 = T.ms0[i], t1 = T.thq1[i];
-    const float2 rp = make_float2(T.ms1[i].w, x1.w);
+    const float4 t1 = T.thq1[i];
+    float4 x1, v1;
+    ldg_record(T.ms, i, x1, v1);
+    const float2 rp = make_float2(v1.w, x1.w);
     const float z = x1.z;
     const int cid = cell_of(P, x1.x, x1.y, z);
     const float pref = snd_eval(P.snd_p, P.snd_n, z).v();
@@ -760,7 +769,7 @@ int af_step(asph_adj* a, StepTape* t) {
     const Bufs own = B;
     if (t) {
         B.nbr = t->lst; B.nbr_cnt = t->cnt;
-        B.ms[0] = t->ms0; B.ms[1] = t->ms1;
+        B.ms = t->ms;
     }
     launch_density(P, B, s);
     if (t) {
@@ -871,13 +880,13 @@ extern "C" int asph_adj_create(asph_ctx* c, int nsteps, int every, asph_adj** ou
 #define AL(p, b) if (e == cudaSuccess) e = a->alloc(&(p), (b))
     for (auto& t : a->tape) {
         AL(t.pos0, N * 16); AL(t.vel0, N * 16); AL(t.thq0, N * 16); AL(t.acc0, N * 16); AL(t.surf0, N);
-        AL(t.perm, N * 4); AL(t.pos1, N * 16); AL(t.ms0, N * 16); AL(t.ms1, N * 16); AL(t.thq1, N * 16);
+        AL(t.perm, N * 4); AL(t.pos1, N * 16); AL(t.ms, N * 32); AL(t.thq1, N * 16);
         AL(t.thq2, N * 16); AL(t.cnt, N * 4); AL(t.lst, (size_t)NBR_CAP * N * 4); AL(t.rain0, C * 4);
         AL(t.dep, C * 4); AL(t.acc, N * 16); AL(t.dthdt, N * 4);
     }
     AdjBufs& A = a->A;
     AL(A.e_pos, N * 16); AL(A.e_vel, N * 16); AL(A.e_thq, N * 16); AL(A.e_acc, N * 16); AL(A.e_rain, C * 4);
-    AL(A.sF, N * 16); AL(A.sV, N * 16); AL(A.lx, N * 16); AL(A.lv, N * 16); AL(A.lq, N * 16);
+    AL(A.sFV, N * 32); AL(A.lx, N * 16); AL(A.lv, N * 16); AL(A.lq, N * 16);
     AL(A.lP, N * 4); AL(A.lS, N * 8); AL(A.l_depc, C * 4); AL(A.l_rain0, C * 4);
     AL(A.ab, 16); AL(A.err, 16);
 #undef AL
@@ -939,9 +948,9 @@ extern "C" int asph_adj_backward(asph_adj* a, const float* dL_dqc, const float* 
     // terminal adjoint: dL/dqc and dL/dtheta of the final state (its order),
     // copied as they are into buffers that the reverse fills later (packing them
     // on the host took 1 ms of a 262k backward)
-    float* const up_qc = reinterpret_cast<float*>(A.sF);
+    float* const up_qc = reinterpret_cast<float*>(A.sFV);
     float* const up_th = up_qc + N;
-    float* const up_xyz = reinterpret_cast<float*>(A.sV);
+    float* const up_xyz = up_th + N;
     if (dL_dqc) CKR(cudaMemcpyAsync(up_qc, dL_dqc, N * 4, cudaMemcpyHostToDevice, s));
     if (dL_dtheta) CKR(cudaMemcpyAsync(up_th, dL_dtheta, N * 4, cudaMemcpyHostToDevice, s));
     if (dL_dxyz) CKR(cudaMemcpyAsync(up_xyz, dL_dxyz, N * 12, cudaMemcpyHostToDevice, s));
@@ -967,7 +976,7 @@ extern "C" int asph_adj_backward(asph_adj* a, const float* dL_dqc, const float* 
     CKR(cudaMemcpyAsync(ab, A.ab, sizeof ab, cudaMemcpyDeviceToHost, s));
     CKR(cudaStreamSynchronize(s));
     if (err) return fail(ASPH_ERR_STATE, "a neighbour list overflowed inside the adjoint window");
-    float* const down = reinterpret_cast<float*>(A.sF);
+    float* const down = reinterpret_cast<float*>(A.sFV);
     k_adj_result<<<blocks(P.N), ATPB, 0, s>>>(P.N, A, down);
     CKR(cudaMemcpyAsync(dL_dtheta0, down, N * 4, cudaMemcpyDeviceToHost, s));
     CKR(cudaStreamSynchronize(s));

@@ -68,6 +68,21 @@ __device__ __forceinline__ float rcp_normal(float x) {
     return r;
 }
 
+// A particle's 32-byte record as one 256-bit access: a neighbour's record is
+// one request and one sector of one line, where two 16-byte arrays are two of
+// each (the gathers of the pair passes run at 65 % of the L1 data pipe).
+__device__ __forceinline__ void ldg_record(const float4* base, int i, float4& a, float4& b) {
+    asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                 : "l"(base + 2 * (size_t)i));
+}
+__device__ __forceinline__ void stg_record(float4* base, int i, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+                 ::"l"(base + 2 * (size_t)i), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z),
+                 "f"(b.w)
+                 : "memory");
+}
+
 // Stop the run from inside a kernel: record the reason (first one wins)
 // and make every later kernel of the step and of later steps do nothing.
 __device__ __forceinline__ void stop_run(DevCtl* ctl, int code) {
@@ -179,8 +194,7 @@ struct DOut {
     const float* rain_cur;
     float* rain_dep;
     const float4* vel;   // velocities the momentum pass reads (after the first half kick) ...
-    float4* ms0;         // ... packed for its neighbour loads: x, y, z, p' ...
-    float4* ms1;         // ... and u, v, w, rho
+    float4* ms;          // ... packed for its neighbour loads: x, y, z, p' and u, v, w, rho
 };
 __device__ __forceinline__ void density_eos_epilogue(const Phys& P, const DOut& O, int i, float4 pi, const DSum& s,
                                                      const FF& rr, float dt) {
@@ -263,8 +277,7 @@ __device__ __forceinline__ void density_eos_epilogue(const Phys& P, const DOut& 
     O.thq[i] = make_float4(th, qv, qc, t.w);
     O.rp[i] = make_float2(rho, ppr);
     const float4 v = O.vel[i];
-    O.ms0[i] = make_float4(pi.x, pi.y, pi.z, ppr);
-    O.ms1[i] = make_float4(v.x, v.y, v.z, rho);
+    stg_record(O.ms, i, make_float4(pi.x, pi.y, pi.z, ppr), make_float4(v.x, v.y, v.z, rho));
 }
 
 // Momentum pair accumulation (asph_h100.cu:448-492), arithmetic rearranged

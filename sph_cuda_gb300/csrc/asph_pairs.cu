@@ -744,9 +744,8 @@ struct MArgs {
     const int2* range;
     const int* nbr;
     const int* nbr_cnt;
-    int use_lists;         // lists (and ms0/ms1) were produced on the current positions and velocities
-    const float4* ms0;     // x, y, z, p' of the density pass
-    const float4* ms1;     // u, v, w, rho of the density pass
+    int use_lists;         // lists (and ms) were produced on the current positions and velocities
+    const float4* ms;      // x, y, z, p' and u, v, w, rho of the density pass, 32 bytes a particle
     MOut out;
     const float* rain_in;
     const float* rain_delta;
@@ -790,8 +789,7 @@ __device__ __forceinline__ void momentum_chunk(const Phys& P, const MArgs& A, in
         // when the lists are current, else from the state buffers
         float4 a, b;
         if (A.use_lists) {
-            a = A.ms0[i];
-            b = A.ms1[i];
+            ldg_record(A.ms, i, a, b);
         } else {
             const float4 p = A.pos[i], v = A.vel[i];
             const float2 rr = A.rp[i];
@@ -818,10 +816,7 @@ __device__ __forceinline__ void momentum_chunk(const Phys& P, const MArgs& A, in
                 for (int u = 0; u < 4; ++u) jj[u] = lp[u * N];
                 lp += 4 * N;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    pp[u] = A.ms0[jj[u]];
-                    vv[u] = A.ms1[jj[u]];
-                }
+                for (int u = 0; u < 4; ++u) ldg_record(A.ms, jj[u], pp[u], vv[u]);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) msum_add(P, s, T, pp[u], vv[u]);
             }
@@ -831,10 +826,7 @@ __device__ __forceinline__ void momentum_chunk(const Phys& P, const MArgs& A, in
 #pragma unroll
                 for (int u = 0; u < 3; ++u) jj[u] = q + u < cnt ? lp[u * N] : i;
 #pragma unroll
-                for (int u = 0; u < 3; ++u) {
-                    pp[u] = A.ms0[jj[u]];
-                    vv[u] = A.ms1[jj[u]];
-                }
+                for (int u = 0; u < 3; ++u) ldg_record(A.ms, jj[u], pp[u], vv[u]);
 #pragma unroll
                 for (int u = 0; u < 3; ++u)
                     if (q + u < cnt) msum_add(P, s, T, pp[u], vv[u]);
@@ -1099,8 +1091,7 @@ void launch_density(const Phys& P, const Bufs& B, cudaStream_t s) {
     A.out.thq = B.thq[B.qc];
     A.out.rp = B.rp;
     A.out.vel = B.vel[B.vc];
-    A.out.ms0 = B.ms[0];
-    A.out.ms1 = B.ms[1];
+    A.out.ms = B.ms;
     const bool reads = P.accretion || P.rain_evap;
     A.out.rain_cur = B.rain[B.rc];
     A.out.rain_dep = reads ? B.rain_delta : B.rain[B.rc];
@@ -1143,8 +1134,7 @@ void launch_momentum(const Phys& P, const Bufs& B, int mode, int use_lists, cuda
     A.nbr = B.nbr;
     A.nbr_cnt = B.nbr_cnt;
     A.use_lists = use_lists;
-    A.ms0 = B.ms[0];
-    A.ms1 = B.ms[1];
+    A.ms = B.ms;
     A.out.thq = B.thq[B.qc];
     A.out.acc = B.acc;
     A.out.dthdt = B.dthdt;
