@@ -913,7 +913,13 @@ int region_cells(const Shape& s, int h) { return (s.bx + 2 * h) * (s.by + 2 * h)
 // times as much as in its brick; under the gated sort they are at most 4 % along an axis
 // (0.3 of one layer in eight), 0.2 % in the runs measured, against 1.6 times the
 // cells to stage.
-int halo_for(const Phys& P) { return P.sort_every <= 1 ? STENCIL : MAX_HALO; }
+// While every target has a resident thread, though, the wider halo is hidden and
+// the deferred kernel would wait for one target's chain of loads (11 us against
+// 4 with nothing queued): density 30.3 -> 28.8 us at 16k, 36.9 -> 34.3 at 65k.
+int halo_for(const Phys& P) {
+    if (P.N <= 152 * 1024) return MAX_HALO;
+    return P.sort_every <= 1 ? STENCIL : MAX_HALO;
+}
 
 // Largest brick whose region fits the grid without wrapping onto itself
 // and whose expected staged count (with a margin) fits the cap.
