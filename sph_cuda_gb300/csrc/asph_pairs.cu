@@ -17,15 +17,16 @@
 // each.  The CTA copies the particles of every table cell within H cells of the
 // brick into shared memory, bucketed row-major by region cell, so that each
 // row of a target's 5 x 5 x 5 window is one contiguous span of slots.  A
-// warp walks its targets' rows together, two candidates a step in fp16, queues
+// warp walks its targets' rows together, four candidates a step in fp16, queues
 // what that test passes in a small per-thread list in shared memory, and
 // drains the lists (float test, density sums, neighbour-list writes) together.
 // What bounds the pass is instruction issue: about 75 candidates and 20
 // neighbours per target at 0.6 particles per cell against 48 bytes.  Density per
 // step at 2M, walk in float with a row advance in every step against this one:
-// 0.6 per cell 511 -> 470 us, the same clustered 1018 -> 830 us, 8:1 cells
-// 516 -> 448 us, one per cell 620 -> 438 us (there with the smaller brick and
-// halo too); 475k 152 -> 135 us, 262k at one per cell 206 -> 147 us.
+// 0.6 per cell 511 -> 466 us, the same clustered 1018 -> 799 us, 8:1 cells
+// 516 -> 436 us, one per cell 1191 -> 741 us (the reference's lattice 620 -> 441;
+// there with the smaller brick and halo too); 475k 152 -> 133 us, 262k at one per cell
+// 206 -> 134 us.
 // H = 2 (the stencil) covers every target still in a cell of its brick; H = 3 also
 // covers one cell of drift since the sort.  A region that overflows the
 // staging capacity is split into its two Morton-aligned halves (each a
@@ -485,9 +486,13 @@ __device__ __forceinline__ void density_region(const Phys& P, const DArgs& A, co
     } while (0)
         const unsigned char* const spb = reinterpret_cast<const unsigned char*>(sp);
         const unsigned char* const gib = reinterpret_cast<const unsigned char*>(s_gidx);
-        // The walk: the window's rows one after another for the whole warp, two
-        // candidates a step, a pair of slots in fp16 (half2: seven
-        // operations for both against ten each in float).  The fp16 test only
+        // The walk: the window's rows one after another for the whole warp, four
+        // candidates a step, two pairs of slots in fp16 (half2: seven
+        // operations for a pair against ten each in float).  The loop's own cost (vote,
+        // branch, queue bound) is a third of a step of one pair, and a row is
+        // mostly two or three pairs: with two pairs a step density takes 466 against
+        // 469 us at 2M, 741 against 822 at one per cell, 799 against 825 clustered
+        // (438 against 441 the other way on the reference's unjittered lattice).  The fp16 test only
         // ever passes too many (FTHR); what passes is queued and takes the float test
         // in the drain.  A lane whose row has ended tests what follows and takes none.
         // Lanes of a warp have rows of much the same length (their windows
@@ -521,33 +526,47 @@ __device__ __forceinline__ void density_region(const Phys& P, const DArgs& A, co
                 int k = kfirst & ~15;
                 while (__any_sync(0xffffffffu, k < kend)) {
                     const uint4 f = *reinterpret_cast<const uint4*>(M.feat + k);
-                    __half2 d = __hsub2(h2_of(f.x), xi2);
-                    __half2 r2 = __hmul2(d, d);
-                    d = __hsub2(h2_of(f.y), yi2);
-                    r2 = __hfma2(d, d, r2);
-                    d = __hsub2(h2_of(f.z), zi2);
-                    r2 = __hfma2(d, d, r2);
+                    const uint4 g = *reinterpret_cast<const uint4*>(M.feat + k + 16);
+                    __half2 d = __hsub2(h2_of(f.x), xi2), e = __hsub2(h2_of(g.x), xi2);
+                    __half2 r2 = __hmul2(d, d), s2 = __hmul2(e, e);
+                    d = __hsub2(h2_of(f.y), yi2); e = __hsub2(h2_of(g.y), yi2);
+                    r2 = __hfma2(d, d, r2); s2 = __hfma2(e, e, s2);
+                    d = __hsub2(h2_of(f.z), zi2); e = __hsub2(h2_of(g.z), zi2);
+                    r2 = __hfma2(d, d, r2); s2 = __hfma2(e, e, s2);
                     asm volatile("{\n"
-                                 "  .reg .pred c, p, q;\n"
-                                 "  .reg .b16 e, o;\n"
-                                 "  setp.lt.s32 c, %3, %6;\n"
-                                 "  setp.le.and.f16x2 p|q, %1, %2, c;\n"
-                                 "  setp.ge.and.s32 p, %3, %4, p;\n"
-                                 "  setp.lt.and.s32 q, %5, %6, q;\n"
-                                 "  cvt.u16.u32 e, %3;\n"
-                                 "  cvt.u16.u32 o, %5;\n"
-                                 "  @p st.shared.u16 [%0], e;\n"
+                                 "  .reg .pred c, p, q, u, v;\n"
+                                 "  .reg .b16 h;\n"
+                                 "  .reg .b32 k1, k2, k3;\n"
+                                 "  add.s32 k1, %4, 8;\n"
+                                 "  add.s32 k2, %4, 16;\n"
+                                 "  add.s32 k3, %4, 24;\n"
+                                 "  setp.lt.s32 c, %4, %6;\n"
+                                 "  setp.le.and.f16x2 p|q, %1, %3, c;\n"
+                                 "  setp.ge.and.s32 p, %4, %5, p;\n"
+                                 "  setp.lt.and.s32 q, k1, %6, q;\n"
+                                 "  setp.lt.s32 c, k2, %6;\n"
+                                 "  setp.le.and.f16x2 u|v, %2, %3, c;\n"
+                                 "  setp.lt.and.s32 v, k3, %6, v;\n"
+                                 "  cvt.u16.u32 h, %4;\n"
+                                 "  @p st.shared.u16 [%0], h;\n"
                                  "  @p add.u32 %0, %0, %7;\n"
-                                 "  @q st.shared.u16 [%0], o;\n"
+                                 "  cvt.u16.u32 h, k1;\n"
+                                 "  @q st.shared.u16 [%0], h;\n"
                                  "  @q add.u32 %0, %0, %7;\n"
+                                 "  cvt.u16.u32 h, k2;\n"
+                                 "  @u st.shared.u16 [%0], h;\n"
+                                 "  @u add.u32 %0, %0, %7;\n"
+                                 "  cvt.u16.u32 h, k3;\n"
+                                 "  @v st.shared.u16 [%0], h;\n"
+                                 "  @v add.u32 %0, %0, %7;\n"
                                  "}\n"
                                  : "+r"(qat)
-                                 : "r"(h2_bits(r2)), "r"(thr), "r"(k), "r"(kfirst), "r"(k + 8), "r"(kend),
+                                 : "r"(h2_bits(r2)), "r"(h2_bits(s2)), "r"(thr), "r"(k), "r"(kfirst), "r"(kend),
                                    "r"(qstep)
                                  : "memory");
-                    k += 16;
-                    room -= 2;
-                    if (room < 2) {   // as far as the steps tell: take the real room, drain when there is little
+                    k += 32;
+                    room -= 4;
+                    if (room < 4) {   // as far as the steps tell: take the real room, drain when there is little
                         room = C.dlist - (int)__umulhi(__reduce_max_sync(0xffffffffu, qat - q0), C.qinv);
                         if (room < 4) {
                             ASPH_DRAIN();
@@ -913,11 +932,13 @@ int region_cells(const Shape& s, int h) { return (s.bx + 2 * h) * (s.by + 2 * h)
 // times as much as in its brick; under the gated sort they are at most 4 % along an axis
 // (0.3 of one layer in eight), 0.2 % in the runs measured, against 1.6 times the
 // cells to stage.
-// While every target has a resident thread, though, the wider halo is hidden and
-// the deferred kernel would wait for one target's chain of loads (11 us against
-// 4 with nothing queued): density 30.3 -> 28.8 us at 16k, 36.9 -> 34.3 at 65k.
+// While the targets are at most half the threads that the GPU holds, though,
+// the wider halo is hidden and the deferred kernel would wait for one target's
+// chain of loads (11 us against 4 with nothing queued): density 30.3 -> 28.8 us at
+// 16k, 36.9 -> 34.3 at 65k.  An ensemble's small members fill the GPU together and pay
+// for it (with the limit at all resident threads, 5.37 -> 5.56 ms for 16 members).
 int halo_for(const Phys& P) {
-    if (P.N <= 152 * 1024) return MAX_HALO;
+    if (P.N <= 152 * 512) return MAX_HALO;
     return P.sort_every <= 1 ? STENCIL : MAX_HALO;
 }
 
