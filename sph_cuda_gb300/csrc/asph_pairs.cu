@@ -51,7 +51,13 @@
 namespace asph {
 
 constexpr int MAX_HALO = 3;      // widest staged halo (cells around a brick)
-constexpr int DENSITY_REGS = 48; // register cap of the brick kernel (its launch plan counts on it)
+// Register cap of the brick kernel (its launch plan counts on it).  48 keep a
+// fourth block of 320 threads per SM, but spill, and leave queues of 18 entries
+// and little staging room; 56 do not spill and leave three blocks queues of 30 and
+// regions that rarely split.  Density with 48 / 56 / 64: 466 / 471 / 470 us at 2M from
+// the lattice, 802 / 693 / 692 clustered, 741 / 728 / 725 at one per cell, 436 / 435 /
+// 466 with 8:1 cells; over 500 steps of the moist bubble 0.964 / 0.941 ms a step.
+constexpr int DENSITY_REGS = 56;
 constexpr int DLIST = 30;        // most queued accepted candidates per thread (D); a launch may use fewer
 // The walk's fp16 test of a candidate.  Coordinates are within FCLAMP < 8
 // cells of the region's centre, so their fp16 rounding is at most 2^-9 each
@@ -585,8 +591,6 @@ __device__ __forceinline__ void density_region(const Phys& P, const DArgs& A, co
     }
 }
 
-// DENSITY_REGS = 48 registers keep 4 blocks of up to 320 threads per SM (the
-// shared-memory limit at the default staging capacity).
 template <int BX, int BY, int BZ, int H>
 __global__ __maxnreg__(DENSITY_REGS) void k_density_brick(const __grid_constant__ Phys P, const __grid_constant__ DArgs A,
                                                        PairCfg C) {
@@ -917,10 +921,10 @@ struct Shape {
 constexpr Shape SHAPES[] = {{8, 8, 8}, {8, 8, 4}, {8, 4, 4}, {4, 4, 4}};
 constexpr int MAX_STAGE = 4096;      // staged particles per brick at most
 constexpr double STAGE_MARGIN = 1.35;
-// Staging capacity that no launch goes below, over the expected count.  1.15 is
-// 1 % faster on an even lattice (465 against 470 us at 2M) and 1.35 leaves a
-// block fewer per SM there (487), but clustered bricks split more often with
-// less (830 us at 1.2, 876 at 1.15).
+// Staging capacity that no launch goes below, over the expected count.  Less
+// splits clustered bricks more often, more can cost a resident block (with 48
+// registers 1.15 / 1.2 / 1.35 took 465 / 470 / 487 us at 2M from the lattice and
+// 876 / 830 / 771 clustered).
 constexpr double STAGE_NEED = 1.2;
 
 int region_cells(const Shape& s, int h) { return (s.bx + 2 * h) * (s.by + 2 * h) * (s.bz + 2 * h); }
