@@ -23,10 +23,11 @@
 // What bounds the pass is instruction issue: about 75 candidates and 20
 // neighbours per target at 0.6 particles per cell against 48 bytes.  Density per
 // step at 2M, walk in float with a row advance in every step against this one:
-// 0.6 per cell 511 -> 466 us, the same clustered 1018 -> 799 us, 8:1 cells
-// 516 -> 436 us, one per cell 1191 -> 741 us (the reference's lattice 620 -> 441;
-// there with the smaller brick and halo too); 475k 152 -> 133 us, 262k at one per cell
-// 206 -> 134 us.
+// 0.6 per cell 511 -> 471 us, the same clustered 1018 -> 693 us, 8:1 cells
+// 516 -> 435 us, one per cell 1191 -> 728 us (the reference's lattice 620 -> 432;
+// there with the smaller brick and halo too); 475k 152 -> 132 us, 262k at one per cell
+// 206 -> 131 us.  It issues on 60 % of the cycles with 31 of 32 lanes, and the
+// shared-memory pipe is busy on 69 % (524k).
 // H = 2 (the stencil) covers every target still in a cell of its brick; H = 3 also
 // covers one cell of drift since the sort.  A region that overflows the
 // staging capacity is split into its two Morton-aligned halves (each a
@@ -496,7 +497,7 @@ __device__ __forceinline__ void density_region(const Phys& P, const DArgs& A, co
         // candidates a step, two pairs of slots in fp16 (half2: seven
         // operations for a pair against ten each in float).  The loop's own cost (vote,
         // branch, queue bound) is a third of a step of one pair, and a row is
-        // mostly two or three pairs: with two pairs a step density takes 466 against
+        // mostly two or three pairs: with two pairs a step (and 48 registers) density takes 466 against
         // 469 us at 2M, 741 against 822 at one per cell, 799 against 825 clustered
         // (438 against 441 the other way on the reference's unjittered lattice).  The fp16 test only
         // ever passes too many (FTHR); what passes is queued and takes the float test
@@ -1038,8 +1039,8 @@ Launch plan(const Phys& P, const Shape& s, int h) {
 // at least SHAPE_WARPS warps resident per SM, and at least four blocks for every
 // SM.  Staged slots and queues, not registers, limit the blocks of a large
 // brick in dense states: at one particle per cell 8 x 8 x 8 cells leave 18 warps per SM
-// and 8 x 8 x 4 leave 36 (density 473 against 433 us at 2M), at 0.6 both leave 40 (466
-// against 569 us); and 112 bricks of 32,768 particles take 88 us where 637 smaller
+// and 8 x 8 x 4 leave 27 (density 473 against 433 us at 2M), at 0.6 both leave 30 (471
+// against 569 us, the latter with 48 registers); and 112 bricks of 32,768 particles take 88 us where 637 smaller
 // ones take 49.  It does not depend on the sort cadence, so the spans that one
 // step's gather wrote serve every other step of the context.
 constexpr int SHAPE_WARPS = 26;
