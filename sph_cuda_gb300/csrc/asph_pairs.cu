@@ -608,20 +608,20 @@ __global__ __maxnreg__(DENSITY_REGS) void k_density_brick(const __grid_constant_
     M.s_list = reinterpret_cast<unsigned short*>(M.s_off + (G::R + 1));
     M.s_warp = s_warp;
     M.s_work = s_work;
+    const int b = blockIdx.x;
+    // the block's two first loads are in flight together, one wait and one barrier less before
+    // its staging starts (ten steps at 2M 7.690 -> 7.669 ms, at 475k 2.147 -> 2.139)
     if (threadIdx.x == 0) {
+        const int bxi = b % C.nbx, byi = (b / C.nbx) % C.nby, bzi = b / (C.nbx * C.nby);
+        const int2 sp2 =
+            A.spans[morton3((uint32_t)(bxi * BX), (uint32_t)(byi * BY), (uint32_t)(bzi * BZ)) >> G::LOG2K];
         s_run = A.ctl->aborted ? 0 : 1;   // one decision per block (barriers follow)
+        s_work[0] = bxi * BX; s_work[1] = byi * BY; s_work[2] = bzi * BZ; s_work[3] = sp2.x; s_work[4] = sp2.y;
         const uint32_t f = h2_bits(__float2half2_rn(1e4f));
         *reinterpret_cast<uint4*>(M.feat + C.cap * 8) = make_uint4(f, f, f, f);
     }
     __syncthreads();
     if (!s_run) return;
-    const int b = blockIdx.x;
-    const int bxi = b % C.nbx, byi = (b / C.nbx) % C.nby, bzi = b / (C.nbx * C.nby);
-    if (threadIdx.x == 0) {
-        const int2 sp2 =
-            A.spans[morton3((uint32_t)(bxi * BX), (uint32_t)(byi * BY), (uint32_t)(bzi * BZ)) >> G::LOG2K];
-        s_work[0] = bxi * BX; s_work[1] = byi * BY; s_work[2] = bzi * BZ; s_work[3] = sp2.x; s_work[4] = sp2.y;
-    }
     density_region<BX, BY, BZ, H, DENSITY_SPLITS>(P, A, C, M, 0);   // (starts with a barrier)
 }
 
