@@ -994,8 +994,10 @@ Launch plan(const Phys& P, const Shape& s, int h) {
     const double ppc = (double)P.N / (double)P.ncell;
     const int R = region_cells(s, h);
     // about one thread per expected target (the lattice keeps brick counts
-    // close to the mean), in whole warps, 64..512
+    // close to the mean), in whole warps, 64..512; a brick of a sparse grid may
+    // expect less than one target
     int groups = (int)(s.bx * s.by * s.bz * ppc * 1.04 + 31) / 32;
+    groups = groups < 1 ? 1 : groups;
     const int rounds = (groups + 15) / 16;
     groups = (groups + rounds - 1) / rounds;
     L.threads = 32 * (groups < 2 ? 2 : groups);
