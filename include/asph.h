@@ -233,8 +233,9 @@ int asph_step_profiled(asph_ctx* ctx, int nsteps, float* phase_ms);
  * ASPH_OPT_TARGETS_PER_THREAD: targets each thread of the momentum pass
  * takes, 1, 2 (default) or 4, so that a warp covers 32, 64 or 128
  * consecutive targets (about 32 k / ppc cells, ppc = particles per cell);
- * 0 restores the default, which takes one where two would leave the GPU
- * short of threads.  Results do not depend on it.
+ * 0 restores the default.  The default takes one where two would leave the
+ * GPU short of threads; get returns the value that is set (2 then as well), and
+ * setting what was read changes nothing.  Results do not depend on it.
  * ASPH_OPT_SORT_AHEAD: 1 (default) = with a sort every step, a run of
  * several steps (asph_step, asph_step_async with nsteps >= 2) sorts the
  * next step's keys beside the current step's density and momentum passes,

@@ -379,7 +379,7 @@ extern "C" int asph_create(const AsphParams* p, void* stream, asph_ctx** out) {
     B.perm = B.vbuf[(B.npasses - 1) & 1];
     B.pc = B.vc = B.qc = B.rc = 0;
     B.shape = -1;
-    B.m_tpt = 0;
+    B.m_tpt = M_TPT;
     cudaStream_t s = c->stream;
     e = cudaMemsetAsync(B.status, 0, (size_t)B.npasses * B.ntiles * 256 * 8, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(B.inc_status, 0, (size_t)B.npasses * B.inc_tiles * 256 * 8, s);
@@ -450,7 +450,7 @@ extern "C" int asph_set_option(asph_ctx* c, int option, int value) {
     } else if (option == ASPH_OPT_TARGETS_PER_THREAD) {
         if (value != 0 && value != 1 && value != 2 && value != 4)
             return fail(ASPH_ERR_ARG, "momentum targets per thread must be 1, 2 or 4 (0: default)");
-        c->B.m_tpt = value;
+        c->B.m_tpt = value ? value : M_TPT;
     } else if (option == ASPH_OPT_SORT_AHEAD) {
         if (value != 0 && value != 1) return fail(ASPH_ERR_ARG, "sort ahead must be 0 or 1");
         c->sort_ahead = value != 0;
@@ -480,7 +480,7 @@ extern "C" int asph_get_option(asph_ctx* c, int option, int* value) {
         return ASPH_OK;
     }
     if (option == ASPH_OPT_TARGETS_PER_THREAD) {
-        *value = momentum_tpt(c->B);
+        *value = c->B.m_tpt;
         return ASPH_OK;
     }
     if (option == ASPH_OPT_SORT_AHEAD) {

@@ -20,6 +20,7 @@ constexpr int sort_tiles(int n) { return (n + sort_tile(n) - 1) / sort_tile(n); 
 constexpr int MAX_PASSES = 4;                      // 30-bit keys / 8-bit digits
 constexpr unsigned SPIN_LIMIT = 1u << 24;          // bounded device waits
 constexpr int NBR_CAP = ASPH_NBR_CAP;              // neighbour-list slots per particle
+constexpr int M_TPT = 2;                           // default of the momentum pass's targets per thread (1, 2 or 4)
 
 // Device-resident step control: the host variables of the reference step
 // loop (asph_h100.cu:931-942, 1040-1078) live here so that a step needs no
@@ -94,7 +95,7 @@ struct Bufs {
     int pc, vc, qc, rc; // current index of pos/vel/thq/rain ping-pong pairs
     int force_global;   // 1: pair passes take the per-target global path, 2: density warp per target
     int shape;          // brick shape index of the density pass, -1: automatic
-    int m_tpt;          // targets per thread of the momentum pass (1, 2 or 4; 0: the default, 2)
+    int m_tpt;          // targets per thread of the momentum pass (1, 2 or 4; M_TPT leaves small launches at 1)
     cudaStream_t aux;   // second stream: the full sort runs beside the incremental one (a graph branch)
     cudaEvent_t ev_fork, ev_join;
     cudaStream_t aux2;  // third stream: the next step's sort beside this step's pair passes
@@ -144,8 +145,6 @@ void sort_inc_sizes(int N, int* max_keys, int* tiles, int* blocks);
 void launch_gather(const Phys& P, const Bufs& B, int mode, cudaStream_t s);
 void launch_density(const Phys& P, const Bufs& B, cudaStream_t s);
 void launch_momentum(const Phys& P, const Bufs& B, int mode, int use_lists, cudaStream_t s);
-// Targets per thread the momentum pass uses (the option, else the default).
-int momentum_tpt(const Bufs& B);
 void launch_rain(const Phys& P, const Bufs& B, cudaStream_t s);
 // Brick shape index the density pass uses (-1: per-target global path),
 // the number of shapes, and whether shape k suits the grid and density.

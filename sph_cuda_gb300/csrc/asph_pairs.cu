@@ -78,7 +78,6 @@ constexpr int M_MINB = 1024 / M_TPB;                     // resident blocks that
 // pass (momentum at 2M from init: 0.262 / 0.245 / 0.256 ms at 256 / 1,024 /
 // 4,096 cells a block).
 constexpr int M_RAIN_CELLS = 8;
-constexpr int M_TPT = 2;         // default targets per thread of the momentum pass (1, 2 or 4 per launch)
 
 template <int BX, int BY, int BZ, int H>
 struct BrickGeom {
@@ -1148,15 +1147,14 @@ void launch_density(const Phys& P, const Bufs& B, cudaStream_t s) {
     }
 }
 
-int momentum_tpt(const Bufs& B) { return B.m_tpt > 0 ? B.m_tpt : M_TPT; }
-// The default takes one target per thread where two would leave the GPU short of
-// threads (152 SMs x 1,024 resident): the lists of a thread's targets are
-// walked one after the other, and with idle SMs that is only latency.  Momentum
-// with one / two: 15.4 / 20.5 us at 16k, 17.4 / 20.5 at 65k, 22.5 / 32.8 at 32k and one
-// per cell, 47.1 / 51.2 at 262k; 59.9 / 59.0 at 475k and 217 / 211 at 2M.
+// The default option value, 2, takes one target per thread where two would leave
+// the GPU short of threads (152 SMs x 1,024 resident): the lists of a thread's
+// targets are walked one after the other, and with idle SMs that is only latency.
+// Momentum with one / two: 15.4 / 20.5 us at 16k, 17.4 / 20.5 at 65k, 22.5 / 32.8 at
+// 32k and one per cell, 47.1 / 51.2 at 262k; 59.9 / 59.0 at 475k and 217 / 211 at 2M.
 static int launch_tpt(const Phys& P, const Bufs& B) {
-    if (B.m_tpt > 0) return B.m_tpt;
-    return P.N <= 2 * 152 * 1024 ? 1 : M_TPT;
+    if (B.m_tpt == M_TPT && P.N <= 2 * 152 * 1024) return 1;
+    return B.m_tpt;
 }
 
 void launch_momentum(const Phys& P, const Bufs& B, int mode, int use_lists, cudaStream_t s) {
