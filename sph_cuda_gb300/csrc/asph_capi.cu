@@ -316,6 +316,7 @@ extern "C" int asph_create(const AsphParams* p, void* stream, asph_ctx** out) {
     asph_ctx* c = new asph_ctx();
     c->prm = *p;
     derive(*p, c->P);
+    cudaGetDevice(&c->device);
     if (stream) {
         c->stream = (cudaStream_t)stream;
     } else {

@@ -12,6 +12,7 @@ struct asph_ctx {
     AsphParams prm;
     Phys P;
     Bufs B{};
+    int device = 0;             // the GPU that was current at asph_create: the buffers and streams are its
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     bool initialised = false;

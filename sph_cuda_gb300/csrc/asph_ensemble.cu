@@ -27,6 +27,7 @@
 // ---------------------------------------------------------------------------
 struct asph_snapshot {
     int N = 0, ncell = 0, nxy = 0;
+    int device = 0;   // the GPU that holds it
     void* mem = nullptr;
     float4 *pos = nullptr, *vel = nullptr, *thq = nullptr, *acc = nullptr;
     float2* rp = nullptr;
@@ -77,6 +78,23 @@ bool same_shape(const asph_ctx* c, const asph_snapshot* s) {
     return s->N == c->P.N && s->ncell == c->P.ncell && s->nxy == c->P.nxy;
 }
 
+// One launch for all parts (see k_copy_parts) where the context, the snapshot and
+// the launch are on one GPU.  Else a copy each: copies carry bytes between the
+// GPUs of a process and may be queued on a stream of a GPU that is not current,
+// where a kernel could neither be launched nor reach the other side.
+int copy_parts(asph_ctx* c, const asph_snapshot* s, const CopyPart* q, int n) {
+    int current = -1;
+    CKR(cudaGetDevice(&current));
+    if (current == c->device && s->device == c->device) {
+        launch_copy_parts(q, n, c->stream);
+        CKR(cudaGetLastError());
+        return ASPH_OK;
+    }
+    for (int k = 0; k < n; ++k)
+        CKR(cudaMemcpyAsync(q[k].dst, q[k].src, q[k].bytes, cudaMemcpyDeviceToDevice, c->stream));
+    return ASPH_OK;
+}
+
 }  // namespace
 
 extern "C" int asph_snapshot_create(asph_ctx* c, asph_snapshot** out) {
@@ -89,7 +107,8 @@ extern "C" int asph_snapshot_create(asph_ctx* c, asph_snapshot** out) {
                                       C * 4, (size_t)s->nxy * 4, sizeof(DevCtl)};
     size_t total = 0;
     for (size_t b : sizes) total += align256(b);
-    cudaError_t e = cudaMalloc(&s->mem, total);
+    cudaError_t e = cudaGetDevice(&s->device);
+    if (e == cudaSuccess) e = cudaMalloc(&s->mem, total);
     if (e != cudaSuccess) {
         delete s;
         return fail(e == cudaErrorMemoryAllocation ? ASPH_ERR_NOMEM : ASPH_ERR_CUDA, "snapshot allocation: %s",
@@ -122,9 +141,7 @@ extern "C" int asph_snapshot_save(asph_ctx* c, asph_snapshot* s) {
     const int n = parts(c, s, p);
     for (int k = 0; k < n; ++k) q[k] = CopyPart{p[k].dev, p[k].snap, p[k].bytes};
     q[n] = CopyPart{c->B.ctl, s->ctl, sizeof(DevCtl)};
-    launch_copy_parts(q, n + 1, c->stream);
-    CKR(cudaGetLastError());
-    return ASPH_OK;
+    return copy_parts(c, s, q, n + 1);
 }
 
 extern "C" int asph_snapshot_restore(asph_ctx* c, const asph_snapshot* s) {
@@ -136,8 +153,8 @@ extern "C" int asph_snapshot_restore(asph_ctx* c, const asph_snapshot* s) {
     for (int k = 0; k < n; ++k) q[k] = CopyPart{p[k].snap, p[k].dev, p[k].bytes};
     // the radix look-back epoch keeps growing (status words of later sorts carry larger epochs)
     q[n] = CopyPart{s->ctl, c->B.ctl, offsetof(DevCtl, epoch)};
-    launch_copy_parts(q, n + 1, c->stream);
-    CKR(cudaGetLastError());
+    const int st = copy_parts(c, s, q, n + 1);
+    if (st) return st;
     c->initialised = true;
     c->lists_valid = false;
     c->spans_valid = false;   // the restored sorted keys' brick spans are rebuilt before the next pass

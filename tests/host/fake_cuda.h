@@ -1,5 +1,6 @@
 // A stand-in for the CUDA runtime calls that a host program of these tests
-// goes through: kernels are recorded and not run.
+// goes through (fake_cuda.cpp): device memory is host memory, copies are made at
+// once and counted, kernels are recorded and not run.
 #pragma once
 #include <cuda_runtime.h>
 #include <vector>
@@ -7,15 +8,12 @@
 struct FakeLaunch {
     dim3 grid, block;
 };
-static std::vector<FakeLaunch> fake_launches;
-
-extern "C" {
-cudaError_t __cudaGetKernel(cudaKernel_t* kernel, const void*) {
-    *kernel = nullptr;
-    return cudaSuccess;
-}
-cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3 grid, dim3 block, void**, size_t, cudaStream_t) {
-    fake_launches.push_back({grid, block});
-    return cudaSuccess;
-}
-}
+struct FakeCopy {
+    const void* src;
+    cudaMemcpyKind kind;
+};
+extern std::vector<FakeLaunch> fake_launches;
+extern std::vector<FakeCopy> fake_copies;   // asynchronous copies and ...
+extern size_t fake_waited;                  // ... how many of them a wait has ended
+extern int fake_device;                     // the current device
+extern bool fake_capture_fails;             // a capture that begins is refused

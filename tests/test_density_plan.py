@@ -6,7 +6,7 @@ import hostbuild
 
 @pytest.fixture(scope="module")
 def plan(tmp_path_factory):
-    return hostbuild.build("plan", tmp_path_factory.mktemp("plan"))
+    return hostbuild.build("plan", tmp_path_factory.mktemp("plan"), fake=False)
 
 
 @pytest.mark.parametrize("n", [1, 60, 64, 125, 1000])
