@@ -935,6 +935,21 @@ extern "C" int asph_adj_forward(asph_adj* a) {
     return ASPH_OK;
 }
 
+namespace {
+
+// Waits for a stream when it goes out of scope, unless that was done already: for
+// a call that may leave early while its copies from or to the caller's arrays (the
+// GPU's own accesses where they are page-locked) are on their way.
+struct WaitOnExit {
+    cudaStream_t s;
+    bool armed = true;
+    ~WaitOnExit() {
+        if (armed) cudaStreamSynchronize(s);
+    }
+};
+
+}  // namespace
+
 extern "C" int asph_adj_backward(asph_adj* a, const float* dL_dqc, const float* dL_dtheta, const float* dL_dxyz,
                                  float* dL_dtheta0, double* dL_dalpha_beta) {
     if (!a || !dL_dtheta0) return fail(ASPH_ERR_ARG, "NULL argument");
@@ -944,7 +959,9 @@ extern "C" int asph_adj_backward(asph_adj* a, const float* dL_dqc, const float* 
     const Phys& P = a->P;
     const size_t N = (size_t)P.N, C = (size_t)P.ncell;
     AdjBufs& A = a->A;
-    int st = ASPH_OK;
+    int st = ASPH_OK, err = 0;
+    double ab[2];
+    WaitOnExit wait{s};
     // terminal adjoint: dL/dqc and dL/dtheta of the final state (its order),
     // copied as they are into buffers that the reverse fills later (packing them
     // on the host took 1 ms of a 262k backward)
@@ -970,8 +987,6 @@ extern "C" int asph_adj_backward(asph_adj* a, const float* dL_dqc, const float* 
         CKR(cudaGetLastError());
     }
     if (st) return st;
-    int err = 0;
-    double ab[2];
     CKR(cudaMemcpyAsync(&err, A.err, sizeof(int), cudaMemcpyDeviceToHost, s));
     CKR(cudaMemcpyAsync(ab, A.ab, sizeof ab, cudaMemcpyDeviceToHost, s));
     CKR(cudaStreamSynchronize(s));
@@ -980,6 +995,7 @@ extern "C" int asph_adj_backward(asph_adj* a, const float* dL_dqc, const float* 
     k_adj_result<<<blocks(P.N), ATPB, 0, s>>>(P.N, A, down);
     CKR(cudaMemcpyAsync(dL_dtheta0, down, N * 4, cudaMemcpyDeviceToHost, s));
     CKR(cudaStreamSynchronize(s));
+    wait.armed = false;
     if (dL_dalpha_beta) {
         dL_dalpha_beta[0] = ab[0];
         dL_dalpha_beta[1] = ab[1];

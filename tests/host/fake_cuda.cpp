@@ -34,6 +34,7 @@ cudaError_t cudaFree(void* p) {
     return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void** p, size_t n) { return cudaMalloc(p, n); }
+cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return cudaMalloc(p, n); }
 cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
 cudaError_t cudaMemcpy(void* dst, const void* src, size_t n, cudaMemcpyKind) {
     memcpy(dst, src, n);
