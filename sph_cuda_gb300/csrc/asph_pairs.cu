@@ -929,13 +929,18 @@ constexpr double STAGE_NEED = 1.2;
 
 int region_cells(const Shape& s, int h) { return (s.bx + 2 * h) * (s.by + 2 * h) * (s.bz + 2 * h); }
 
-// Staged halo: with a sort every step, or the displacement-gated sort (at
-// most 0.3 cells of drift along each axis), few targets have left their brick, and the
-// stencil alone is staged; slower cadences stage one more cell of drift.
-// Targets outside either go to the deferred pass, where one costs two to three
-// times as much as in its brick; under the gated sort they are at most 4 % along an axis
-// (0.3 of one layer in eight), 0.2 % in the runs measured, against 1.6 times the
-// cells to stage.
+// Staged halo: with a sort every step, or the displacement-gated sort (about
+// 0.3 cells of the fastest target's way and the last step's own), few targets have
+// left their brick, and the stencil alone is staged; slower cadences stage one more
+// cell of drift.  Targets outside either go to the deferred pass, where one costs two
+// to three times as much as in its brick.  Under the gated sort these are, just
+// before a sort and if every target moves as fast as the fastest, 3.75 % of a
+// brick along an axis of 8 cells and 7.5 % along one of 4; in the runs measured
+// 0.2 %.  Density with no drift / averaged over a gated interval of such a flow along
+// one axis / two / three, against the wide halo: 485 / 585 / 656 / 793 against 679 us
+// at 2M and one per cell (8x8x4), 471 / 545 / 608 / 668 against 630 at 0.6 per cell
+// (8x8x8), 51 / 61 / 65 / 68 against 64 at 98k (8x4x4).  A floor and a lid keep the third
+// axis out of that.
 // While the targets are at most half the threads that the GPU holds, though,
 // the wider halo is hidden and the deferred kernel would wait for one target's
 // chain of loads (11 us against 4 with nothing queued): density 30.3 -> 28.8 us at
