@@ -1047,16 +1047,23 @@ Launch plan(const Phys& P, const Shape& s, int h) {
 // brick in dense states: at one particle per cell 8 x 8 x 8 cells leave 18 warps per SM
 // and 8 x 8 x 4 leave 27 (density 473 against 433 us at 2M), at 0.6 both leave 30 (471
 // against 569 us, the latter with 48 registers); and 112 bricks of 32,768 particles take 88 us where 637 smaller
-// ones take 49.  It does not depend on the sort cadence, so the spans that one
-// step's gather wrote serve every other step of the context.
+// ones take 49.  A smaller brick is taken for its warps only while it has more of them:
+// on a sparse grid (below 0.16 per cell) the eight blocks of two warps are all
+// there are, and smaller bricks only add blocks (a step at 0.03 per cell on 100 x 100
+// x 100 cells: 72 us with 8 x 8 x 8, 177 with 4 x 4 x 4).  The choice does not depend on the
+// sort cadence, so the spans that one step's gather wrote serve every other step of
+// the context.
 constexpr int SHAPE_WARPS = 26;
 int pick_shape(const Phys& P) {
     int k = 0;
     while (k < 4 && !fits(P, k)) ++k;
     if (k == 4) return -1;
+    Launch L = plan(P, SHAPES[k], STENCIL);
     for (; k < 3; ++k) {
-        const Launch L = plan(P, SHAPES[k], STENCIL);
-        if (L.blocks * (L.threads / 32) >= SHAPE_WARPS && L.C.nbricks >= 4 * 152) break;
+        const Launch next = plan(P, SHAPES[k + 1], STENCIL);
+        const int warps = L.blocks * (L.threads / 32), more = next.blocks * (next.threads / 32);
+        if ((warps >= SHAPE_WARPS || more <= warps) && L.C.nbricks >= 4 * 152) break;
+        L = next;
     }
     return k;
 }

@@ -16,3 +16,16 @@ def test_sparse_grids_have_a_plan(plan, grid, n):
     r = hostbuild.run(plan, *grid, n)
     assert r.returncode == 0, "exit %d" % r.returncode
     assert -1 <= int(r.stdout) <= 3
+
+
+@pytest.mark.parametrize("grid,n,shape", [
+    # sparse: smaller bricks would be no better filled, only more
+    ((100, 100, 100), 3000, 0), ((100, 100, 100), 30000, 0), ((100, 100, 100), 150000, 0), ((160, 160, 160), 40960, 0),
+    # few bricks: smaller ones until every SM has four
+    ((64, 64, 64), 7864, 1), ((40, 40, 40), 28800, 3),
+    # dense: smaller ones while they leave more warps resident
+    ((133, 133, 200), 2097152, 0), ((128, 128, 128), 2097152, 1),
+])
+def test_shape_for_the_density_of_the_grid(plan, grid, n, shape):
+    r = hostbuild.run(plan, *grid, n)
+    assert r.returncode == 0 and int(r.stdout) == shape
