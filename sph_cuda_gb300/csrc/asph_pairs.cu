@@ -946,8 +946,13 @@ int region_cells(const Shape& s, int h) { return (s.bx + 2 * h) * (s.by + 2 * h)
 // chain of loads (11 us against 4 with nothing queued): density 30.3 -> 28.8 us at
 // 16k, 36.9 -> 34.3 at 65k.  An ensemble's small members fill the GPU together and pay
 // for it (with the limit at all resident threads, 5.37 -> 5.56 ms for 16 members).
-int halo_for(const Phys& P) {
-    if (P.N <= 152 * 512) return MAX_HALO;
+// That needs the bricks resident together, eight per SM: on a sparse grid of more
+// bricks the staging is most of the pass (a step with 40,960 particles on 160 x 160 x 160
+// cells, 8,000 bricks: 188 us with the wide halo, 172 without).
+int halo_for(const Phys& P, const Shape& s) {
+    const long long bricks =
+        (long long)((P.nx + s.bx - 1) / s.bx) * ((P.ny + s.by - 1) / s.by) * ((P.nz + s.bz - 1) / s.bz);
+    if (P.N <= 152 * 512 && bricks <= 152 * 8) return MAX_HALO;
     return P.sort_every <= 1 ? STENCIL : MAX_HALO;
 }
 
@@ -1091,7 +1096,7 @@ void launch_dh(const Phys& P, const DArgs& A, cudaStream_t s) {
 
 template <int BX, int BY, int BZ>
 void launch_d(const Phys& P, const DArgs& A, cudaStream_t s) {
-    if (halo_for(P) == STENCIL) launch_dh<BX, BY, BZ, STENCIL>(P, A, s);
+    if (halo_for(P, Shape{BX, BY, BZ}) == STENCIL) launch_dh<BX, BY, BZ, STENCIL>(P, A, s);
     else launch_dh<BX, BY, BZ, MAX_HALO>(P, A, s);
 }
 

@@ -155,3 +155,26 @@ def test_gated_sorts_above_the_wide_halos_size(shape, brick):
             used = np.arange(lst.shape[0])[:, None] < np.maximum(cnt, 0)[None, :]
             assert np.array_equal(lst[used], lst_g[used])
         assert between >= 3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,grid,narrow", [(30000, (100, 100, 100), True), (30000, (64, 64, 64), False)])
+def test_wide_halo_only_while_the_bricks_are_resident_together(n, grid, narrow):
+    """Few targets on a grid of many bricks: the halo to stage is then most of the pass."""
+    drift = 0.25
+    p = small_config(lat=(n, 1, 1), grid=grid, box=tuple(g * c for g, c in zip(grid, (200.0, 200.0, 50.0))), sort_every=1)
+    s = random_state(p, 9, "uniform")
+    for f in ("u", "v", "w", "ax", "ay", "az"):
+        s[f] = np.zeros(n, np.float32)
+    with Asph(p) as sim:
+        s["u"][:] = drift * 200.0 / sim.control()["dt"]
+        sim.set_state(s)
+        sim.sort_build()
+        sim.kick_drift_flux()
+        sim.density_eos()
+        deferred = sim.control()["deferred"]
+    left = drift / 8 * n   # uniform positions: the share of an 8-cell edge within `drift` of its end
+    if narrow:
+        assert 0.85 * left < deferred < 1.15 * left   # five standard deviations of a count of 938
+    else:
+        assert deferred == 0
