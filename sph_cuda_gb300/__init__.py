@@ -239,7 +239,8 @@ class Asph:
         return v.value
 
     def set_targets_per_thread(self, k: int) -> None:
-        """Momentum-pass targets per thread: 1, 2 or 4 (a warp covers 32 k targets)."""
+        """Momentum-pass targets per thread: 1, 2 or 4 (a warp covers 32 k targets).  2 is the
+        default, which takes one where two would leave the GPU short of threads."""
         _check(self.lib.asph_set_option(self._ctx, abi.OPT_TARGETS_PER_THREAD, int(k)))
 
     def sort_ahead(self) -> bool:

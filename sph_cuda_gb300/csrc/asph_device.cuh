@@ -49,9 +49,8 @@ __device__ __forceinline__ float r2_pair(const Phys& P, float xi, float yi, floa
     return __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmul_rn(dz, dz)));
 }
 
-// Reciprocal and reciprocal square root of the pair sums, without the
-// subnormal handling that rsqrtf and __fdividef carry (four to six
-// instructions each): their arguments are normal numbers by construction
+// Reciprocal and reciprocal square root of the pair sums, without subnormal
+// handling: their arguments are normal numbers by construction
 // (densities >= 1e-3, r^2 >= 1e-30, r^2 + eta^2 > 0), for which the results are
 // the same bits.  Both pair passes are bound by instruction issue and by
 // latency: density 613.6 -> 573.9 us and momentum 267.5 -> 252.5 us on a 128^3

@@ -504,8 +504,9 @@ __device__ __forceinline__ void density_region(const Phys& P, const DArgs& A, co
         // Lanes of a warp have rows of much the same length (their windows
         // overlap), so waiting for the longest one costs less than letting each
         // lane run on into its next row, a dozen instructions more in every step.
-        // The next row's span is read one row ahead (a chain of latencies where few warps
-        // are left: 893 -> 876 us in the clustered state, 504 -> 466 even).
+        // The next row's span is read one row ahead: 893 -> 876 us clustered and 504 -> 466 even
+        // with one pair a step and 48 registers; with two pairs and 56 it makes no difference
+        // (468 against 468 us at 2M, 960 against 956 clustered without it).
         const __half2 xi2 = __half2half2(feat_coord(pi.x, cx, P.inv_dx));
         const __half2 yi2 = __half2half2(feat_coord(pi.y, cy0, P.inv_dy));
         const __half2 zi2 = __half2half2(feat_coord(pi.z, cz, P.inv_dz));
@@ -920,7 +921,7 @@ struct Shape {
 };
 constexpr Shape SHAPES[] = {{8, 8, 8}, {8, 8, 4}, {8, 4, 4}, {4, 4, 4}};
 constexpr int MAX_STAGE = 4096;      // staged particles per brick at most
-constexpr double STAGE_MARGIN = 1.35;
+constexpr double STAGE_MARGIN = 1.35;   // of the expected region count, in fits(): which shapes a grid admits
 // Staging capacity that no launch goes below, over the expected count.  Less
 // splits clustered bricks more often, more can cost a resident block (with 48
 // registers 1.15 / 1.2 / 1.35 took 465 / 470 / 487 us at 2M from the lattice and
@@ -945,7 +946,7 @@ int region_cells(const Shape& s, int h) { return (s.bx + 2 * h) * (s.by + 2 * h)
 // the wider halo is hidden and the deferred kernel would wait for one target's
 // chain of loads (11 us against 4 with nothing queued): density 30.3 -> 28.8 us at
 // 16k, 36.9 -> 34.3 at 65k.  An ensemble's small members fill the GPU together and pay
-// for it (with the limit at all resident threads, 5.37 -> 5.56 ms for 16 members).
+// for it (with the limit at all resident threads, 4.87 -> 5.01 ms for 16 members).
 // That needs the bricks resident together, eight per SM: on a sparse grid of more
 // bricks the staging is most of the pass (a step with 40,960 particles on 160 x 160 x 160
 // cells, 8,000 bricks: 188 us with the wide halo, 172 without).
@@ -1013,7 +1014,7 @@ Launch plan(const Phys& P, const Shape& s, int h) {
     auto smem_for = [&](size_t cap, int dlist) {
         return cap * (8 + 16 + 4) + 16 + (size_t)4 * (R + 1) + (size_t)dlist * L.threads * 2;
     };
-    // staging capacity: at least the expected region count times STAGE_MARGIN;
+    // staging capacity: at least the expected region count times STAGE_NEED;
     // the most resident blocks the registers allow come first, then the
     // deepest drain queue (fuller drains) that still fits them, then all the
     // shared memory left for staging, so that clustered bricks overflow less

@@ -25,7 +25,7 @@ CASES = {
     "clustered": (lambda: small_config(lat=(40, 40, 20), grid=(40, 40, 40), box=(8000.0, 8000.0, 2000.0)), "cluster"),
     # pairs across the periodic edge, whose raw distances are a box length
     "anisotropic_wide": (lambda: _wide(), "jitter"),
-    # more targets than the device has resident threads at two blocks of 512 per SM (77,824):
+    # more than 77,824 targets, one block of 512 threads per SM:
     # sorted every step the narrow halo, which drifted targets leave; every fourth step the wide one
     "narrow_halo": (lambda: small_config(lat=(48, 42, 42), grid=(48, 42, 40), box=(9600.0, 8400.0, 2000.0),
                                          sort_every=1), "jitter"),
